@@ -21,6 +21,7 @@
 #include <cmath>
 #include <string>
 
+#include "reduce_dev.cuh"
 #include "sop_dev.cuh"
 #include "../../include/sop_gpu.h"
 
@@ -31,6 +32,7 @@ constexpr int kThreads = 256;
 constexpr int kItemsPerThread = 4;
 constexpr int kMaxBlocks = 4096;
 constexpr long long kMaxItems = (long long)kMaxBlocks * kThreads * kItemsPerThread;
+constexpr int kFinalThreads = 256;
 
 // Partial sums of the four energy terms, one group of four per block.  Each
 // call writes the partials of every block it launches before the final sum
@@ -63,19 +65,21 @@ __device__ __forceinline__ void separation(const float* x, int i, int j, float b
 
 __device__ __forceinline__ bool bead_ok(int i, int nbead) { return i >= 0 && i < nbead; }
 
-// One thread per list entry over [bonds | angles | native pairs | non-native
-// pairs]; the same FP32 terms as k_energy, summed in FP64 per block.  An
+// A thread takes kItemsPerThread list entries, kThreads apart (a warp reads
+// consecutive entries), of [bonds | angles | native pairs | non-native pairs];
+// the same FP32 terms as k_energy, summed in FP64 per block.  An
 // entry whose bead index lies outside [0, nbead), or whose bead type is not
 // 1 or 2, is not evaluated: it adds NaN to its term, so the caller sees the
 // bad input in that term and in rna_etot instead of an out-of-bounds read.
 __global__ void __launch_bounds__(kThreads) k_energy_lists(Lists L, double* __restrict__ scratch) {
-  __shared__ double red[4][kThreads / 32];
+  __shared__ double red[4 * 32];
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   const double bad = __longlong_as_double(0x7ff8000000000000LL);  // quiet NaN
   const long long n1 = L.nbnd, n2 = n1 + L.nang, n3 = n2 + L.natt, n4 = n3 + L.nrep;
-  const long long base = ((long long)blockIdx.x * kThreads + threadIdx.x) * kItemsPerThread;
+  const long long base = (long long)blockIdx.x * kThreads * kItemsPerThread + threadIdx.x;
+#pragma unroll
   for (int q = 0; q < kItemsPerThread; ++q) {
-    const long long e = base + q;
+    const long long e = base + q * kThreads;
     if (e >= n4) break;
     float dx, dy, dz, lx, ly, lz;
     if (e < n1) {
@@ -116,33 +120,28 @@ __global__ void __launch_bounds__(kThreads) k_energy_lists(Lists L, double* __re
       acc[3] += (double)(L.rep6 ? L.eps_rep * u3 : L.eps_rep * u3 * (u3 + 1.0f));
     }
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    double v = acc[t];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[t][w] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double v = 0.0;
-    for (int k = 0; k < kThreads / 32; ++k) v += red[threadIdx.x][k];
-    scratch[4 * blockIdx.x + threadIdx.x] = v;
-  }
+  const double x = block_sums<4>(acc, red);
+  if (threadIdx.x < 4) scratch[4 * blockIdx.x + threadIdx.x] = x;
 }
 
-// Final FP64 sum of the partials in block order (e_bnd gets -(k R0^2 / 2),
-// energy.cu:223), then rna_etot (energy.cu:76).
-__global__ void k_energy_lists_final(const double* __restrict__ scratch, int nblocks,
-                                     double bnd_coeff, double* __restrict__ out) {
+// Final FP64 sum of the partials (e_bnd gets -(k R0^2 / 2), energy.cu:223),
+// then rna_etot (energy.cu:76).  One block; a thread per term took 23 us at 484
+// partials, the loads one after another.
+__global__ void __launch_bounds__(kFinalThreads) k_energy_lists_final(const double* __restrict__ scratch,
+                                                                       int nblocks, double bnd_coeff,
+                                                                       double* __restrict__ out) {
+  __shared__ double red[4 * 32];
   __shared__ double t[4];
+  pdl_wait();
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblocks; b += kFinalThreads)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] += scratch[4 * b + k];
+  double x = block_sums<4>(v, red);
   if (threadIdx.x < 4) {
-    double v = 0.0;
-    for (int b = 0; b < nblocks; ++b) v += scratch[4 * b + threadIdx.x];
-    if (threadIdx.x == 0) v *= -bnd_coeff;
-    t[threadIdx.x] = v;
-    out[threadIdx.x] = v;
+    if (threadIdx.x == 0) x *= -bnd_coeff;
+    t[threadIdx.x] = x;
+    out[threadIdx.x] = x;
   }
   __syncthreads();
   if (threadIdx.x == 0) out[4] = t[0] + t[1] + t[2] + t[3];
@@ -213,7 +212,8 @@ int sop_energy_noalloc(const sop_params* p, const sop_energy_lists* l, double* t
   const int nb = (int)std::max<long long>(1, (items + per_block - 1) / per_block);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   k_energy_lists<<<nb, kThreads, 0, st>>>(L, scratch);
-  k_energy_lists_final<<<1, 32, 0, st>>>(scratch, nb, 0.5 * p->k_bnd * p->R0 * p->R0, terms);
+  launch_pdl(k_energy_lists_final, 1, kFinalThreads, st, (const double*)scratch, nb,
+             0.5 * p->k_bnd * p->R0 * p->R0, terms);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     g_err = std::string("sop_energy_noalloc: launch: ") + cudaGetErrorString(e);

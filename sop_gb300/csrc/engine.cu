@@ -51,6 +51,7 @@ void launch_step_tiles(const DevSys& s, int koff, bool step, const int4* tiles, 
                        bool any_split, cudaStream_t st);
 void launch_advance(const DevSys& s, int steps, cudaStream_t st);
 void launch_gather_current(const DevSys& s, float* out, int* flag_out, cudaStream_t st);
+int energy_blocks(int mol_n);
 void launch_energy(const DevSys& s, int mol_start, int mol_n, int m, double* part, double* out,
                    double k_bnd_R0sq_half, cudaStream_t st);
 void launch_observables(const DevSys& s, int mol_start, int mol_n, int m, int nnat,
@@ -757,7 +758,7 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   ctx->w.ncell = ctx->dalloc<int>(nm);
   ctx->w.block_sums = ctx->dalloc<int>(scan_block_sums_needed(std::max<long long>(c.cells, nb)));
   ctx->w.cells_total = ctx->dalloc<int>(1);
-  ctx->e_part = ctx->dalloc<double>(6 * ((size_t)c.max_mol_beads / 256 + 2));
+  ctx->e_part = ctx->dalloc<double>(6 * (size_t)energy_blocks((int)c.max_mol_beads));
   ctx->e_out = ctx->dalloc<double>(8);
   if (!s.x[0] || !s.x[1] || !s.p[0] || !s.p[1] || !s.v || !s.incr || !s.f || !s.fsum || !s.mol_of ||
       !s.mol || !s.mol_step || !s.mol_status || !s.sys_step || !s.bond_row || !s.ang_row ||

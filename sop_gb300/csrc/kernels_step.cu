@@ -20,6 +20,7 @@
 // to track parity, and every molecule may sit at its own step.
 #include <algorithm>
 
+#include "reduce_dev.cuh"
 #include "sop_dev.cuh"
 #include "../../include/sop_gpu.h"
 
@@ -709,9 +710,18 @@ __global__ void k_advance(DevSys s, int steps) {
 // Per-bead FP32 terms over the bead's full rows (each pair counted from both
 // beads, so halved), reduced in FP64: e_bnd, e_ang_ss, e_vdw_att, e_vdw_rep
 // (energy.cu:194-225, 278-307, 369-442).  Partial sums per block.
-__global__ void __launch_bounds__(256) k_energy(DevSys s, int mol_start, int mol_n, int m,
-                                                 double* __restrict__ part) {
-  __shared__ double red[4][8];
+//
+// A bead's terms are added one after another in row order, in FP32, so its
+// sums do not depend on the launch; the loads and the terms of kTermBatch
+// entries are independent and in flight together (one entry at a time, the
+// chain index -> coordinates -> divide took about 600 cycles an entry: 47 us
+// at 50,000 beads, 15 us at any small size).
+constexpr int kEnergyThreads = 128;
+constexpr int kTermBatch = 4;
+
+__global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, int mol_start, int mol_n, int m,
+                                                            double* __restrict__ part) {
+  __shared__ double red[4 * 32];
   int i = mol_start + blockIdx.x * blockDim.x + threadIdx.x;
   float eb = 0.f, ea = 0.f, eat = 0.f, erp = 0.f;
   if (i < mol_start + mol_n) {
@@ -736,60 +746,72 @@ __global__ void __launch_bounds__(256) k_energy(DevSys s, int mol_start, int mol
       const float4 xj = X[s.ang_j[ar.x + e]];
       float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
       min_image3(dx, dy, dz, boxl);
-      float inv = 1.0f / (dx * dx + dy * dy + dz * dz);
-      ea += s.e_ss * inv * inv * inv;
+      float inv = 1.0f / __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+      ea = __fmaf_rn(__fmul_rn(__fmul_rn(s.e_ss, inv), inv), inv, ea);
     }
     const int abase = s.nat_row[i].x, acnt = s.pl_att_cnt[i];
-    for (int e = 0; e < acnt; ++e) {
-      const float4 q = s.pl_att[abase + e];
-      const float4 xj = X[__float_as_int(q.x)];
-      float lx, ly, lz;
-      float dx = diff_exact(xj.x, xi.x, lx), dy = diff_exact(xj.y, xi.y, ly),
-            dz = diff_exact(xj.z, xi.z, lz);
-      min_image3(dx, dy, dz, boxl);
-      float d2 = dx * dx + dy * dy + dz * dz;
-      float sr = q.y * q.y / d2;
-      float s3 = sr * sr * sr;
-      float sm1 = -d2_minus_r02(dx, dy, dz, lx, ly, lz, q.y) / d2;
-      // eps_e (s^6 - 2 s^3) = eps_e (s^3 (s^3 - 1) - s^3)
-      eat += q.w * (s3 * sm1 * (sr * sr + sr + 1.0f) - s3);
+    for (int e0 = 0; e0 < acnt; e0 += kTermBatch) {
+      float4 q[kTermBatch], xx[kTermBatch];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) q[c] = s.pl_att[abase + min(e0 + c, acnt - 1)];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) xx[c] = X[__float_as_int(q[c].x)];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) {
+        if (e0 + c >= acnt) break;
+        float lx, ly, lz;
+        float dx = diff_exact(xx[c].x, xi.x, lx), dy = diff_exact(xx[c].y, xi.y, ly),
+              dz = diff_exact(xx[c].z, xi.z, lz);
+        min_image3(dx, dy, dz, boxl);
+        float d2 = dx * dx + dy * dy + dz * dz;
+        float sr = q[c].y * q[c].y / d2;
+        float s3 = sr * sr * sr;
+        float sm1 = -d2_minus_r02(dx, dy, dz, lx, ly, lz, q[c].y) / d2;
+        // eps_e (s^6 - 2 s^3) = eps_e (s^3 (s^3 - 1) - s^3)
+        eat += q[c].w * (s3 * sm1 * (sr * sr + sr + 1.0f) - s3);
+      }
     }
     const long long rbase = (long long)i * s.nl_stride;
     const int rcnt = s.pl_cnt[i];
     const int ti = type_of(xi);
     const int jbase = s.mol[m].start;
-    for (int e = 0; e < rcnt; ++e) {
-      const float4 xj = X[jbase + (int)s.pl_j[rbase + e]];
-      float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-      min_image3(dx, dy, dz, boxl);
-      float u = s.sig2[ti][type_of(xj)] / (dx * dx + dy * dy + dz * dz);
-      float u3 = u * u * u;
-      erp += s.rep6 ? s.eps_rep * u3 : s.eps_rep * u3 * (u3 + 1.0f);
+    for (int e0 = 0; e0 < rcnt; e0 += kTermBatch) {
+      float4 xx[kTermBatch];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c)
+        xx[c] = X[jbase + (int)s.pl_j[rbase + min(e0 + c, rcnt - 1)]];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) {
+        if (e0 + c >= rcnt) break;
+        float dx = xx[c].x - xi.x, dy = xx[c].y - xi.y, dz = xx[c].z - xi.z;
+        min_image3(dx, dy, dz, boxl);
+        float u = pick_type_pair(s.sig2[1][1], s.sig2[1][2], s.sig2[2][2], ti, type_of(xx[c])) /
+                  (dx * dx + dy * dy + dz * dz);
+        float u3 = u * u * u;
+        erp += s.rep6 ? s.eps_rep * u3 : s.eps_rep * u3 * (u3 + 1.0f);
+      }
     }
   }
   double v[4] = {0.5 * (double)eb, 0.5 * (double)ea, 0.5 * (double)eat, 0.5 * (double)erp};
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    double x = v[t];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[t][w] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double x = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) x += red[threadIdx.x][k];
-    part[4 * blockIdx.x + threadIdx.x] = x;
-  }
+  const double x = block_sums<4>(v, red);
+  if (threadIdx.x < 4) part[4 * blockIdx.x + threadIdx.x] = x;
 }
 
-// Final FP64 sum of the per-block partials, in block order.
-__global__ void k_energy_final(const double* __restrict__ part, int nblocks, double k_bnd_R0sq_half,
-                               double* __restrict__ out) {
+// Final FP64 sum of the per-block partials: a block of 256 threads (one
+// thread per term took 12 us at 196 partials, the loads one after another).
+constexpr int kFinalThreads = 256;
+
+__global__ void __launch_bounds__(kFinalThreads) k_energy_final(const double* __restrict__ part,
+                                                                 int nblocks, double k_bnd_R0sq_half,
+                                                                 double* __restrict__ out) {
+  __shared__ double red[4 * 32];
+  pdl_wait();
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblocks; b += kFinalThreads)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] += part[4 * b + t];
+  double x = block_sums<4>(v, red);
   if (threadIdx.x >= 4) return;
-  double x = 0.0;
-  for (int b = 0; b < nblocks; ++b) x += part[4 * b + threadIdx.x];
   if (threadIdx.x == 0) x *= -k_bnd_R0sq_half;  // e_bnd = -(k R0^2 / 2) sum log(...)
   out[threadIdx.x] = x;
 }
@@ -798,55 +820,63 @@ __global__ void k_energy_final(const double* __restrict__ part, int nblocks, dou
 // Q over all native contacts (each counted from its lower bead), the
 // first and second moments of the coordinates for Rg^2, and sum v^2, in FP64
 // (sop.cu:528-611).  Partials per block: {contacts, sx, sy, sz, sxx, svv}.
-__global__ void __launch_bounds__(256) k_observables(DevSys s, int mol_start, int mol_n, int m,
-                                                      double* __restrict__ part) {
-  __shared__ double red[6][8];
+__global__ void __launch_bounds__(kEnergyThreads) k_observables(DevSys s, int mol_start, int mol_n,
+                                                                 int m, double* __restrict__ part) {
+  __shared__ double red[8 * 32];
   int i = mol_start + blockIdx.x * blockDim.x + threadIdx.x;
-  double v[6] = {0, 0, 0, 0, 0, 0};
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (i < mol_start + mol_n) {
     const int cur = (int)(s.mol_step[m] & 1);
     const float4* X = s.x[cur];
     const float4 xi = X[i];
+    const float4 vi = s.v[i];
     const int2 nr = s.nat_row[i];
     int cnt = 0;
-    for (int e = 0; e < nr.y; ++e) {
-      int j = s.nat_j[nr.x + e];
-      if (j < i) continue;
-      const float4 xj = X[j];
-      float dx = __fsub_rn(xi.x, xj.x), dy = __fsub_rn(xi.y, xj.y),
-            dz = __fsub_rn(xi.z, xj.z);
-      min_image3(dx, dy, dz, s.boxl);
-      float d = sqrtf(d2_exact(dx, dy, dz));
-      if (__fdiv_rn(d, s.nat_par[nr.x + e].x) < 1.25f) ++cnt;
+    for (int e0 = 0; e0 < nr.y; e0 += kTermBatch) {
+      int j[kTermBatch];
+      float4 xx[kTermBatch];
+      float r0[kTermBatch];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) {
+        const int e = nr.x + min(e0 + c, nr.y - 1);
+        j[c] = s.nat_j[e];
+        r0[c] = s.nat_par[e].x;
+      }
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) xx[c] = X[j[c]];
+#pragma unroll
+      for (int c = 0; c < kTermBatch; ++c) {
+        float dx = __fsub_rn(xi.x, xx[c].x), dy = __fsub_rn(xi.y, xx[c].y),
+              dz = __fsub_rn(xi.z, xx[c].z);
+        min_image3(dx, dy, dz, s.boxl);
+        const float d = sqrtf(d2_exact(dx, dy, dz));
+        if (e0 + c < nr.y && j[c] >= i && __fdiv_rn(d, r0[c]) < 1.25f) ++cnt;
+      }
     }
-    const float4 vi = s.v[i];
     v[0] = cnt;
     v[1] = xi.x; v[2] = xi.y; v[3] = xi.z;
     v[4] = (double)xi.x * xi.x + (double)xi.y * xi.y + (double)xi.z * xi.z;
     v[5] = (double)vi.x * vi.x + (double)vi.y * vi.y + (double)vi.z * vi.z;
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < 6; ++t) {
-    double x = v[t];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[t][w] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    double x = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) x += red[threadIdx.x][k];
-    part[6 * blockIdx.x + threadIdx.x] = x;
-  }
+  const double x = block_sums<8>(v, red);
+  if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = x;
 }
 
-__global__ void k_observables_final(const double* __restrict__ part, int nblocks, int n, int nnat,
-                                    double* __restrict__ out) {
+// (A single thread took 55 us over 196 blocks' partials.)
+__global__ void __launch_bounds__(kFinalThreads) k_observables_final(const double* __restrict__ part,
+                                                                      int nblocks, int n, int nnat,
+                                                                      double* __restrict__ out) {
+  __shared__ double red[8 * 32];
+  __shared__ double t[8];
+  pdl_wait();
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nblocks; b += kFinalThreads)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] += part[6 * b + k];
+  const double x = block_sums<8>(v, red);
+  if (threadIdx.x < 8) t[threadIdx.x] = x;
+  __syncthreads();
   if (threadIdx.x != 0) return;
-  double t[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int k = 0; k < 6; ++k) t[k] += part[6 * b + k];
   const double inv = 1.0 / n;
   const double mx = t[1] * inv, my = t[2] * inv, mz = t[3] * inv;
   out[0] = nnat ? t[0] / nnat : 0.0;                           // Q
@@ -1063,18 +1093,21 @@ void launch_advance(const DevSys& s, int steps, cudaStream_t st) {
   launch_pdl(k_advance, cdiv(s.nmol, 256), 256, st, s, steps);
 }
 
+// Blocks (and groups of partial sums) of an energy or observables launch.
+int energy_blocks(int mol_n) { return (int)cdiv(mol_n, kEnergyThreads); }
+
 void launch_energy(const DevSys& s, int mol_start, int mol_n, int m, double* part, double* out,
                    double k_bnd_R0sq_half, cudaStream_t st) {
-  int nb = (int)cdiv(mol_n, 256);
-  k_energy<<<nb, 256, 0, st>>>(s, mol_start, mol_n, m, part);
-  k_energy_final<<<1, 32, 0, st>>>(part, nb, k_bnd_R0sq_half, out);
+  const int nb = energy_blocks(mol_n);
+  k_energy<<<nb, kEnergyThreads, 0, st>>>(s, mol_start, mol_n, m, part);
+  launch_pdl(k_energy_final, 1, kFinalThreads, st, (const double*)part, nb, k_bnd_R0sq_half, out);
 }
 
 void launch_observables(const DevSys& s, int mol_start, int mol_n, int m, int nnat, double* part,
                         double* out, cudaStream_t st) {
-  int nb = (int)cdiv(mol_n, 256);
-  k_observables<<<nb, 256, 0, st>>>(s, mol_start, mol_n, m, part);
-  k_observables_final<<<1, 32, 0, st>>>(part, nb, mol_n, nnat, out);
+  const int nb = energy_blocks(mol_n);
+  k_observables<<<nb, kEnergyThreads, 0, st>>>(s, mol_start, mol_n, m, part);
+  launch_pdl(k_observables_final, 1, kFinalThreads, st, (const double*)part, nb, mol_n, nnat, out);
 }
 
 }  // namespace sop
