@@ -184,12 +184,16 @@ def whole_job_rate(beads_per_rank: int, md_steps: int, world: int, t_max: float)
     return world * beads_per_rank * md_steps / t_max
 
 
-def launches_per_bench_step(p, s0: int, form: int = 1) -> int:
+def launches_per_bench_step(p, s0: int, form: int = 1, beads: int = 0, largest: int = 0) -> int:
     """Kernels of the engine in one replay starting after step s0 (form 1:
     one step kernel per step; 2: force + finish kernels; 3 and 4: one
-    launch per run of steps between list rebuilds)."""
-    nl_kernels = 12    # bbox reset, bbox, grid, grid base, assign, 3 scan, scatter, cellsort,
-                       # stage_xs, nl
+    launch per run of steps between list rebuilds), in a context of `beads`
+    beads whose largest molecule has `largest`."""
+    nl_kernels = 2     # bin_mol, nl
+    if beads > 16384:
+        nl_kernels += 1    # att
+    if largest > 8192:
+        nl_kernels += 10   # bbox reset, bbox, grid, assign, 3 scan, scatter, cellsort, stage_xs
     n = 0
     runs = 0
     in_run = False
@@ -421,7 +425,7 @@ def plain_measure(workload: str, local: int, K: int, warmup: int, lanes: int = 0
     tuning = e.tuning()
     e.close()
     s0 = stages[names[0]]
-    n_launch = sum(launches_per_bench_step(p, s_start + k * MD_STEPS, tuning["form"])
+    n_launch = sum(launches_per_bench_step(p, s_start + k * MD_STEPS, tuning["form"], mol.n, mol.n)
                    for k in range(K))
     cpu = None
     if cpu_seconds > 0:
@@ -609,6 +613,7 @@ def main() -> None:
         e.step_async(MD_STEPS)
     e.sync()
     s_start = [eng.status(0)[1] for eng in e.engines]
+    part_sizes = [[m.n for m in eng.mols] for eng in e.engines]
     tuning = e.tuning()
 
     K = args.steps
@@ -727,8 +732,9 @@ def main() -> None:
         served = served_stream(local)
 
     if rank == 0:
-        n_launch = sum(launches_per_bench_step(p, s0_ + k * MD_STEPS, tu.get("form", 1))
-                       for s0_, tu in zip(s_start, tuning) for k in range(K))
+        n_launch = sum(launches_per_bench_step(p, s0_ + k * MD_STEPS, tu.get("form", 1), sum(ns),
+                                               max(ns))
+                       for s0_, tu, ns in zip(s_start, tuning, part_sizes) for k in range(K))
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_max / K, "higher_is_better": True,

@@ -28,9 +28,8 @@
 namespace sop {
 // kernels_lists.cu
 struct NLScratch {
-  int* ncell;
   int* block_sums;
-  int* cells_total;
+  int min_mol, max_mol;
 };
 void launch_nl_rebuild(const DevSys& s, const NLScratch& w, int koff, cudaStream_t st);
 void launch_pl_rebuild(const DevSys& s, int koff, cudaStream_t st);
@@ -79,7 +78,7 @@ struct HostMol {
 // Capacities of the device pools.
 struct Caps {
   long long beads = 0, mols = 0, bonds = 0, angles = 0, natives = 0, cells = 0;
-  long long max_mol_beads = 0, stride = 64;
+  long long max_mol_beads = 0, min_mol_beads = 1, stride = 64;
 };
 
 // First-fit allocator of ranges in [0, cap), coalescing on release.
@@ -746,8 +745,10 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   s.bbox = ctx->dalloc<unsigned>(6 * nm);
   s.grid = ctx->dalloc<MolGrid>(nm);
   s.cell_cap = c.cells;
-  s.cell_cnt = ctx->dalloc<int>(c.cells);
   s.cell_start = ctx->dalloc<int>(c.cells + 1);
+  const long long chain = c.max_mol_beads > kBinMolBeads ? c.cells + 1 : 0;
+  s.cell_cnt = ctx->dalloc<int>(chain);
+  s.cell_scan = ctx->dalloc<int>(chain);
   s.bead_cell = ctx->dalloc<int>(nb);
   s.bead_slot = ctx->dalloc<int>(nb);
   s.sorted = ctx->dalloc<int>(nb);
@@ -755,9 +756,9 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   s.flags = ctx->dalloc<int>(4);  // [0] flags, [2..3] the persistent step's barrier
   s.noise = nullptr;
   s.use_noise = 0;
-  ctx->w.ncell = ctx->dalloc<int>(nm);
+  ctx->w.min_mol = (int)c.min_mol_beads;
+  ctx->w.max_mol = (int)c.max_mol_beads;
   ctx->w.block_sums = ctx->dalloc<int>(scan_block_sums_needed(std::max<long long>(c.cells, nb)));
-  ctx->w.cells_total = ctx->dalloc<int>(1);
   ctx->e_part = ctx->dalloc<double>(6 * (size_t)energy_blocks((int)c.max_mol_beads));
   ctx->e_out = ctx->dalloc<double>(8);
   if (!s.x[0] || !s.x[1] || !s.p[0] || !s.p[1] || !s.v || !s.incr || !s.f || !s.fsum || !s.mol_of ||
@@ -765,8 +766,8 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
       !s.nat_row || !s.bond_j || !s.bond_r0 || !s.ang_j || !s.nat_j || !s.nat_par ||
       !s.nat_rc2 || !s.nl_att_cnt || !s.pl_att_cnt || !s.nl_att_e || !s.pl_att || !s.nl_cnt ||
       !s.pl_cnt || !s.nl_maxrow || !s.bbox || !s.grid || !s.cell_cnt || !s.cell_start ||
-      !s.bead_cell || !s.bead_slot || !s.sorted || !s.xs || !s.flags || !ctx->w.ncell ||
-      !ctx->w.block_sums || !ctx->w.cells_total || !ctx->e_part || !ctx->e_out)
+      !s.cell_scan || !s.bead_cell || !s.bead_slot || !s.sorted || !s.xs || !s.flags ||
+      !ctx->w.block_sums || !ctx->e_part || !ctx->e_out)
     return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
   if (!ctx->h_out) CK(cudaMallocHost(&ctx->h_out, 8 * sizeof(double)));
   cudaStream_t st = ctx->stream;
@@ -782,8 +783,6 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   CK(cudaMemsetAsync(s.pl_att_cnt, 0, sizeof(int) * nb, st));
   CK(cudaMemsetAsync(s.nl_cnt, 0, sizeof(int) * nb, st));
   CK(cudaMemsetAsync(s.pl_cnt, 0, sizeof(int) * nb, st));
-  CK(cudaMemsetAsync(s.cell_cnt, 0, sizeof(int) * (size_t)c.cells, st));
-  CK(cudaMemsetAsync(s.cell_start, 0, sizeof(int) * (size_t)(c.cells + 1), st));  // nothing binned yet
   CK(cudaMemsetAsync(s.bond_row, 0, sizeof(int2) * nb, st));
   CK(cudaMemsetAsync(s.ang_row, 0, sizeof(int2) * nb, st));
   CK(cudaMemsetAsync(s.nat_row, 0, sizeof(int2) * nb, st));
@@ -1176,10 +1175,11 @@ int commit(SopCtx* ctx) {
     c.bonds += 2LL * (long long)m.bi.size();
     c.angles += 2LL * (long long)m.ai.size();
     c.natives += 2LL * (long long)m.ni.size();
-    c.cells += std::max<long long>(64, 2LL * m.n);
     c.max_mol_beads = std::max<long long>(c.max_mol_beads, m.n);
+    c.min_mol_beads = &m == &ctx->mols[0] ? m.n : std::min<long long>(c.min_mol_beads, m.n);
   }
   c.mols = (long long)ctx->mols.size();
+  c.cells = 3 * c.beads;
   if (c.beads <= 0) return ctx->fail(SOP_ERR_ARG, "no beads");
   // rows sized so that most contexts never regrow them (a regrowth costs a
   // second list build at commit); a longer row regrows from the first
@@ -1748,7 +1748,7 @@ int sop_serve_create(const sop_params* p, long long budget_bytes, long long max_
   c.bonds = 2 * c.beads;
   c.angles = 2 * c.beads;
   c.natives = 8 * c.beads;
-  c.cells = 2 * c.beads + 64 * c.mols;
+  c.cells = 3 * c.beads;
   c.max_mol_beads = max_job_beads;
   c.stride = stride;
   rc = alloc_pools(ctx, c);

@@ -3,20 +3,23 @@
 // sort + scan they use).
 //
 // Neighbour list (every nnlup steps):
-//   1. per-molecule bounding box of the coordinates             k_bbox
-//   2. per-molecule cell grid (cell edge rc/S, S=1..3 chosen so a cell holds
-//      ~4 beads; S=1..4 and ~1 bead from 10,000 beads up; molecules whose
-//      extent + rc reaches boxl, where the minimum image matters, fall back
-//      to index-chunked cells that scan all pairs)
-//                                                                k_grid, k_grid_base
-//   3. counting sort of beads into cells (own scan), cells sorted by bead id
-//      so every later order is deterministic, coordinates staged in that
-//      order                             k_assign, scan, k_scatter, k_cellsort, k_stage_xs
-//   4. 8 lanes per bead in cell order: the bead against the beads of the
-//      cell rows within S along each axis, culled to its own cut-off sphere;
-//      predicate = the reference's FP32 host filter (d^2 < rcut^2, |i-j| > 2,
-//      not native); one pass writes fixed-stride rows (overflow: regrow) k_nl
-//   The attractive neighbour list filters each bead's native row (k_assign).
+//   1. binning: each molecule's bounding box, its cell grid (cell edge rc/S,
+//      S=1..3 chosen so a cell holds ~4 beads; S=1..4 and ~1 bead from 10,000
+//      beads up; molecules whose extent + rc reaches boxl, where the minimum
+//      image matters, fall back to index-chunked cells that scan all pairs), a
+//      counting sort of its beads into cells, cells sorted by bead id so every
+//      later order is deterministic, coordinates staged in that order.  A
+//      molecule's cells start at cell_base and its staged beads at its first
+//      bead, so molecules are binned independently: one block per molecule,
+//      in shared memory (k_bin_mol); molecules past kBinMolBeads by a chain of
+//      kernels over all their beads (k_bbox, k_grid, k_assign, scan,
+//      k_scatter, k_cellsort, k_stage_xs)
+//   2. 8 lanes (or a warp) per bead in cell order: the bead against the beads
+//      of the cell rows within S along each axis, culled to its own cut-off
+//      sphere; predicate = the reference's FP32 host filter (d^2 < rcut^2,
+//      |i-j| > 2, not native); one pass writes fixed-stride rows (overflow:
+//      regrow).  The attractive neighbour list filters the bead's native row.
+//                                                                          k_nl
 // Pair list (every nplup steps): eight lanes per bead, beads in chain order,
 // compact its neighbour-list row in row order (k_pl).
 #include "sop_dev.cuh"
@@ -110,16 +113,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
 }
 
 // ---------------------------------------------------------------- grids
-// Each binning kernel's work per item is a device function, so that the
-// kernels below and the one-block binning of small contexts (k_bin_small)
-// share it.
-__device__ __forceinline__ void bbox_reset_at(const DevSys& s, int m) {
-  if (m >= s.nmol) return;
-  unsigned* b = s.bbox + 6 * m;
-  b[0] = b[1] = b[2] = f2ord(INFINITY);
-  b[3] = b[4] = b[5] = f2ord(-INFINITY);
-}
-__global__ void k_bbox_reset(DevSys s) { bbox_reset_at(s, blockIdx.x * blockDim.x + threadIdx.x); }
+// First cell of the molecule whose beads start at `start`.  A molecule of n
+// beads has at most 2 n cells (n / 32 chunks when every pair is scanned) and
+// one more entry of cell_start, which 3 n hold, so the ranges of molecules are
+// apart wherever their beads are.
+__device__ __forceinline__ int cell_base(int start) { return 3 * start; }
 
 // Molecules whose lists a rebuild at block offset koff refreshes: running,
 // healthy, and with the step this rebuild precedes (mol_step + koff + 1)
@@ -138,10 +136,22 @@ __device__ __forceinline__ const float4* xbuf(const DevSys& s, int m, int koff) 
   return s.x[(int)((s.mol_step[m] + koff) & 1)];
 }
 
-// Called by all 32 lanes of a warp together (warp votes).
-__device__ __forceinline__ void bbox_at(const DevSys& s, int koff, int i) {
+__device__ __forceinline__ bool bins_by_chain(const DevSys& s, int m, int koff) {
+  return mol_listed(s, m, koff) && s.mol[m].n > kBinMolBeads;
+}
+
+__global__ void k_bbox_reset(DevSys s) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= s.nmol) return;
+  unsigned* b = s.bbox + 6 * m;
+  b[0] = b[1] = b[2] = f2ord(INFINITY);
+  b[3] = b[4] = b[5] = f2ord(-INFINITY);
+}
+
+__global__ void k_bbox(DevSys s, int koff) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int m = (i < s.nlive) ? s.mol_of[i] : -1;
-  bool ok = mol_listed(s, m, koff);
+  bool ok = bins_by_chain(s, m, koff);
   unsigned act = __ballot_sync(0xffffffffu, ok);
   if (!ok) return;
   float4 x = xbuf(s, m, koff)[i];
@@ -162,30 +172,15 @@ __device__ __forceinline__ void bbox_at(const DevSys& s, int koff, int i) {
     }
   }
 }
-__global__ void k_bbox(DevSys s, int koff) { bbox_at(s, koff, blockIdx.x * blockDim.x + threadIdx.x); }
 
-// One thread per molecule: cell grid of its neighbour-list build.
-__device__ __forceinline__ void grid_at(const DevSys& s, int* ncell, int koff, int m) {
-  if (m >= s.nmol) return;
-  if (s.only_mol >= 0 && m != s.only_mol) {  // a rebuild of another molecule alone
-    ncell[m] = 0;
-    return;
-  }
+// The cell grid of a molecule of n beads within the bounds b (ordered floats:
+// three lower, three upper).
+__device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsigned* b, int base) {
   MolGrid g = {};
-  int n = s.mol[m].n;
-  if (!mol_listed(s, m, koff) || n <= 0) {
-    g.ncell = 0;
-    s.grid[m] = g;
-    ncell[m] = 0;
-    return;
-  }
-  // the bounds come from atomics (performed in L2): read them from L2, so
-  // that a block that reset them itself cannot see its own stale L1 lines
-  const unsigned* b = s.bbox + 6 * m;
   float lo[3], ext[3];
   for (int a = 0; a < 3; ++a) {
-    lo[a] = ord2f(__ldcg(b + a));
-    ext[a] = ord2f(__ldcg(b + 3 + a)) - lo[a];
+    lo[a] = ord2f(b[a]);
+    ext[a] = ord2f(b[3 + a]) - lo[a];
   }
   const float rc = s.rc_nl_rep_max;
   bool periodic = false;
@@ -197,12 +192,7 @@ __device__ __forceinline__ void grid_at(const DevSys& s, int* ncell, int koff, i
   bool wrap = false;
   for (int a = 0; a < 3; ++a) wrap |= !(ext[a] + rc < 0.25f * s.boxl);
   if (periodic || n <= 96) {
-    // every pair is scanned; cells are chunks of 32 consecutive beads
     g.brute = 1;
-    g.dims[0] = (n + 31) / 32; g.dims[1] = 1; g.dims[2] = 1;
-    g.S = g.dims[0];
-    g.cs = 0.0f;
-    g.lo[0] = g.lo[1] = g.lo[2] = 0.0f;
   } else {
     float vol = fmaxf((ext[0] + 1.0f) * (ext[1] + 1.0f) * (ext[2] + 1.0f), 1.0f);
     float rho = (float)n / vol;
@@ -214,9 +204,10 @@ __device__ __forceinline__ void grid_at(const DevSys& s, int* ncell, int koff, i
     int S = (int)floorf(rc * cbrtf(rho * (big ? 1.0f : 0.25f)));
     S = S < 1 ? 1 : (S > smax ? smax : S);
     float cs = rc * 1.0001f / (float)S + 1.0e-4f;
-    long long cap = n * 2 > 64 ? (long long)n * 2 : 64;
-    for (int iter = 0; iter < 8; ++iter) {
-      long long tot = 1;
+    const long long cap = 2LL * n;
+    long long tot = 0;
+    for (int iter = 0; iter < 64; ++iter) {
+      tot = 1;
       for (int a = 0; a < 3; ++a) {
         g.dims[a] = (int)floorf(ext[a] / cs) + 1;
         tot *= g.dims[a];
@@ -226,42 +217,22 @@ __device__ __forceinline__ void grid_at(const DevSys& s, int* ncell, int koff, i
       S = (int)ceilf(rc * 1.0001f / cs);
       if (S < 1) S = 1;
     }
-    g.brute = 0;
     g.S = S;
     g.cs = cs;
     for (int a = 0; a < 3; ++a) g.lo[a] = lo[a];
+    g.brute = tot > cap;  // a bound on the cells, not reached: each round takes 1% off at least
+  }
+  if (g.brute) {
+    // every pair is scanned; cells are chunks of 32 consecutive beads
+    g.dims[0] = (n + 31) / 32; g.dims[1] = 1; g.dims[2] = 1;
+    g.S = g.dims[0];
+    g.cs = 0.0f;
+    g.lo[0] = g.lo[1] = g.lo[2] = 0.0f;
   }
   g.wrap = wrap ? 1 : 0;
   g.ncell = g.dims[0] * g.dims[1] * g.dims[2];
-  s.grid[m] = g;
-  ncell[m] = g.ncell;
-}
-__global__ void k_grid(DevSys s, int* __restrict__ ncell, int koff) {
-  grid_at(s, ncell, koff, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// Single block: cell bases = exclusive scan of the per-molecule cell counts;
-// flags overflow of the cell capacity (cannot happen by construction: each
-// molecule holds at most max(64, 2n) cells, and the capacity is their sum).
-// Called by every thread of one block.
-__device__ __forceinline__ void grid_base_block(const DevSys& s, const int* ncell, int* cells_total) {
-  int carry = 0;
-  for (int b0 = 0; b0 < s.nmol; b0 += blockDim.x) {
-    int m = b0 + threadIdx.x;
-    int v = m < s.nmol ? ncell[m] : 0;
-    int total;
-    int ex = block_excl_scan(v, &total);
-    if (m < s.nmol) s.grid[m].base = ex + carry;
-    carry += total;
-  }
-  if (threadIdx.x == 0) {
-    if (carry > s.cell_cap) atomicOr(s.flags, FLAG_NL_OVERFLOW);
-    *cells_total = carry > s.cell_cap ? (int)s.cell_cap : carry;
-  }
-}
-__global__ void __launch_bounds__(1024) k_grid_base(DevSys s, const int* __restrict__ ncell,
-                                                     int* __restrict__ cells_total) {
-  grid_base_block(s, ncell, cells_total);
+  g.base = base;
+  return g;
 }
 
 __device__ __forceinline__ int cell_coord(float v, float lo, float cs, int dim) {
@@ -269,129 +240,174 @@ __device__ __forceinline__ int cell_coord(float v, float lo, float cs, int dim) 
   return c < 0 ? 0 : (c >= dim ? dim - 1 : c);
 }
 
-// Per bead: cell index and slot (counting sort), plus the attractive
-// neighbour-list filter of its native row (sop.cu:704-759 semantics).
-__device__ __forceinline__ void assign_at(const DevSys& s, int koff, int att, int i) {
-  if (i >= s.nlive) return;
-  int m = s.mol_of[i];
-  if (!mol_listed(s, m, koff)) {  // not binned; its lists stay as they are
-    s.bead_cell[i] = -1;
-    return;
-  }
-  const float4* X = xbuf(s, m, koff);
-  float4 xi = X[i];
-  MolGrid g = s.grid[m];
-  int c;
-  if (g.brute) {
-    c = g.base + (i - s.mol[m].start) / 32;
-  } else {
-    int cx = cell_coord(xi.x, g.lo[0], g.cs, g.dims[0]);
-    int cy = cell_coord(xi.y, g.lo[1], g.cs, g.dims[1]);
-    int cz = cell_coord(xi.z, g.lo[2], g.cs, g.dims[2]);
-    c = g.base + (cz * g.dims[1] + cy) * g.dims[0] + cx;
-  }
-  if (c < 0 || c >= s.cell_cap) {  // unreachable: capacity is the sum of the per-molecule caps
-    atomicOr(s.flags, FLAG_NL_OVERFLOW);
-    s.bead_cell[i] = -1;
-    s.nl_att_cnt[i] = 0;
-    return;
-  }
-  s.bead_cell[i] = c;
-  s.bead_slot[i] = atomicAdd(s.cell_cnt + c, 1);
-  if (!att) return;  // binning only: the lists stay as they are
-  int2 row = s.nat_row[i];
-  int k = 0;
-  for (int e = 0; e < row.y; ++e) {
-    int idx = row.x + e;
-    float4 xj = X[s.nat_j[idx]];
-    float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y),
-          dz = __fsub_rn(xj.z, xi.z);
-    min_image3(dx, dy, dz, s.boxl);
-    if (d2_exact(dx, dy, dz) < s.nat_rc2[idx].x) s.nl_att_e[row.x + k++] = idx;
-  }
-  s.nl_att_cnt[i] = k;
-}
-__global__ void k_assign(DevSys s, int koff, int att) {
-  assign_at(s, koff, att, blockIdx.x * blockDim.x + threadIdx.x);
+// The cell of a bead (r within its molecule) at x, within its molecule's grid.
+__device__ __forceinline__ int cell_of(const MolGrid& g, int r, float4 x) {
+  if (g.brute) return r / 32;
+  const int cx = cell_coord(x.x, g.lo[0], g.cs, g.dims[0]);
+  const int cy = cell_coord(x.y, g.lo[1], g.cs, g.dims[1]);
+  const int cz = cell_coord(x.z, g.lo[2], g.cs, g.dims[2]);
+  return (cz * g.dims[1] + cy) * g.dims[0] + cx;
 }
 
-__device__ __forceinline__ void scatter_at(const DevSys& s, int i) {
-  if (i >= s.nlive) return;
-  int c = s.bead_cell[i];
-  if (c < 0) return;
-  s.sorted[s.cell_start[c] + s.bead_slot[i]] = i;
-}
-__global__ void k_scatter(DevSys s) { scatter_at(s, blockIdx.x * blockDim.x + threadIdx.x); }
-
-// Per cell: sort its beads by id (fixes every downstream order).  Cells hold
-// a handful of beads, so one thread's insertion sort is short.
-__device__ __forceinline__ void cellsort_at(const DevSys& s, const int* cells_total, long long c) {
-  if (c >= *cells_total) return;
-  int cnt = __ldcg(s.cell_cnt + c);  // counted by atomics: read from L2
-  if (cnt == 0) return;
-  int* b = s.sorted + s.cell_start[c];
+// Insertion sort of a cell's beads by id (fixes every downstream order).
+// Cells hold a handful of beads, so one thread's sort is short.
+__device__ __forceinline__ void sort_cell(int* b, int cnt) {
   for (int a = 1; a < cnt; ++a) {
     int v = b[a], k = a;
     while (k > 0 && b[k - 1] > v) { b[k] = b[k - 1]; --k; }
     b[k] = v;
   }
 }
-__global__ void k_cellsort(DevSys s, const int* __restrict__ cells_total) {
-  cellsort_at(s, cells_total, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+
+// ------------------------------------------------- one block per molecule
+// Blocks walk the molecule slots (a served context has many free ones: each
+// thread looks at one slot, the block then bins the live ones in turn).  The
+// cell counts, their scan and the sorted order stay in shared memory; a
+// chain of 11 launches with its counts in L2, or one block for the whole
+// context, took 145-158 us for 1,500-13,000 beads and 69 us for 4,000.
+__global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) {
+  extern __shared__ int bin_smem[];
+  int* first = bin_smem;                                // cells: counts, then first position
+  int* order = bin_smem + 2 * most + 1;        // beads in cell order
+  __shared__ unsigned bounds[6];
+  __shared__ MolGrid grid;
+  __shared__ int found[1024];
+  __shared__ int nfound;
+  const int T = blockDim.x, t = threadIdx.x, lane = t & 31;
+  for (long long m0 = blockIdx.x; m0 < s.nmol; m0 += (long long)gridDim.x * T) {
+    if (t == 0) nfound = 0;
+    __syncthreads();
+    const long long mt = m0 + (long long)t * gridDim.x;
+    if (mt < s.nmol && mol_listed(s, (int)mt, koff) && s.mol[mt].n <= kBinMolBeads)
+      found[atomicAdd(&nfound, 1)] = (int)mt;
+    __syncthreads();
+    for (int f = 0; f < nfound; ++f) {
+      const int m = found[f];
+      const int n = s.mol[m].n, start = s.mol[m].start;
+      const float4* X = xbuf(s, m, koff) + start;
+      if (t < 6) bounds[t] = t < 3 ? f2ord(INFINITY) : f2ord(-INFINITY);
+      __syncthreads();
+      unsigned mn[3], mx[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = f2ord(INFINITY);
+        mx[a] = f2ord(-INFINITY);
+      }
+      for (int r = t; r < n; r += T) {
+        const float4 x = X[r];
+        const unsigned o[3] = {f2ord(x.x), f2ord(x.y), f2ord(x.z)};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          mn[a] = min(mn[a], o[a]);
+          mx[a] = max(mx[a], o[a]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
+        mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          atomicMin(bounds + a, mn[a]);
+          atomicMax(bounds + 3 + a, mx[a]);
+        }
+      }
+      __syncthreads();
+      if (t == 0) {
+        grid = make_grid(s, n, bounds, cell_base(start));
+        s.grid[m] = grid;
+      }
+      __syncthreads();
+      const int ncell = grid.ncell;
+      for (int c = t; c < ncell; c += T) first[c] = 0;
+      __syncthreads();
+      for (int r = t; r < n; r += T) {
+        const int c = cell_of(grid, r, X[r]);
+        s.bead_cell[start + r] = grid.base + c;
+        s.bead_slot[start + r] = atomicAdd(first + c, 1);
+      }
+      __syncthreads();
+      // exclusive scan: a run of cells per thread
+      const int per = (ncell + T - 1) / T, c0 = min(t * per, ncell), c1 = min(c0 + per, ncell);
+      int sum = 0;
+      for (int c = c0; c < c1; ++c) sum += first[c];
+      int total;
+      int at = block_excl_scan(sum, &total);
+      for (int c = c0; c < c1; ++c) {
+        const int v = first[c];
+        first[c] = at;
+        at += v;
+      }
+      if (t == 0) first[ncell] = n;
+      __syncthreads();
+      for (int r = t; r < n; r += T)
+        order[first[s.bead_cell[start + r] - grid.base] + s.bead_slot[start + r]] = r;
+      __syncthreads();
+      for (int c = t; c <= ncell; c += T) {
+        if (c < ncell) sort_cell(order + first[c], first[c + 1] - first[c]);
+        s.cell_start[grid.base + c] = start + first[c];
+      }
+      __syncthreads();
+      for (int k = t; k < n; k += T) {
+        const int r = order[k];
+        float4 x = X[r];
+        x.w = __int_as_float(((start + r) << 2) | type_of(x));
+        s.xs[start + k] = x;
+      }
+      __syncthreads();  // the next molecule reuses the shared memory
+    }
+    __syncthreads();
+  }
+}
+
+// ------------------------------------- the chain, for molecules past that
+// Cell counts in cell_cnt, their exclusive scan over all cells in cell_scan;
+// a molecule's beads then lie in the order of its cells at
+// cell_scan - cell_scan[its first cell] past its first bead.
+__global__ void k_grid(DevSys s, int koff) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= s.nmol || !bins_by_chain(s, m, koff)) return;
+  unsigned b[6];
+  for (int a = 0; a < 6; ++a) b[a] = s.bbox[6 * m + a];
+  s.grid[m] = make_grid(s, s.mol[m].n, b, cell_base(s.mol[m].start));
+}
+
+__global__ void k_assign(DevSys s, int koff) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.nlive) return;
+  const int m = s.mol_of[i];
+  if (!bins_by_chain(s, m, koff)) return;
+  const MolGrid g = s.grid[m];
+  const int c = g.base + cell_of(g, i - s.mol[m].start, xbuf(s, m, koff)[i]);
+  s.bead_cell[i] = c;
+  s.bead_slot[i] = atomicAdd(s.cell_cnt + c, 1);
+}
+
+__global__ void k_scatter(DevSys s, int koff) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.nlive || !bins_by_chain(s, s.mol_of[i], koff)) return;
+  s.sorted[s.cell_scan[s.bead_cell[i]] + s.bead_slot[i]] = i;
+}
+
+__global__ void k_cellsort(DevSys s) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= s.cell_cap) return;
+  const int cnt = s.cell_cnt[c];
+  if (cnt > 1) sort_cell(s.sorted + s.cell_scan[c], cnt);
 }
 
 // Coordinates staged in cell order, w = (id << 2) | type: a thread per
 // position, so the gathers are independent.
-__device__ __forceinline__ void stage_xs_at(const DevSys& s, int koff, int k) {
-  if (k >= s.cell_start[s.cell_cap]) return;  // beads that were binned
+__global__ void k_stage_xs(DevSys s, int koff) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= s.cell_scan[s.cell_cap]) return;  // beads that were binned
   const int i = s.sorted[k];
-  float4 x = xbuf(s, s.mol_of[i], koff)[i];
+  const int m = s.mol_of[i];
+  float4 x = xbuf(s, m, koff)[i];
   x.w = __int_as_float((i << 2) | type_of(x));
-  s.xs[k] = x;
-}
-__global__ void k_stage_xs(DevSys s, int koff) { stage_xs_at(s, koff, blockIdx.x * blockDim.x + threadIdx.x); }
-
-// The whole binning in one block, for contexts small enough that the chain of
-// kernels above costs mostly launch latency: the same per-item work, phase
-// by phase, with block barriers between phases, so the same cells, order
-// and coordinates.  The scan of the cell counts runs over the block.
-constexpr int kBinThreads = 1024;
-constexpr long long kBinSmallCells = 1 << 16;
-//
-// Values that atomics produced in this kernel (the molecule bounds, the cell
-// counts) are read with __ldcg: atomics complete in L2, and the block's own
-// L1 may still hold the lines it cleared before them.
-__global__ void __launch_bounds__(kBinThreads) k_bin_small(DevSys s, int* ncell, int* cells_total,
-                                                           int koff, int att) {
-  const int t = threadIdx.x;
-  for (int m = t; m < s.nmol; m += kBinThreads) bbox_reset_at(s, m);
-  __syncthreads();
-  // every lane of a warp takes part in each round (warp votes)
-  for (int i0 = 0; i0 < s.nlive; i0 += kBinThreads) bbox_at(s, koff, i0 + t);
-  __syncthreads();
-  for (int m = t; m < s.nmol; m += kBinThreads) grid_at(s, ncell, koff, m);
-  __syncthreads();
-  grid_base_block(s, ncell, cells_total);
-  for (long long c = t; c < s.cell_cap; c += kBinThreads) s.cell_cnt[c] = 0;
-  __syncthreads();
-  for (int i = t; i < s.nlive; i += kBinThreads) assign_at(s, koff, att, i);
-  __syncthreads();
-  int carry = 0;  // exclusive scan of the cell counts into cell_start
-  for (long long c0 = 0; c0 < s.cell_cap; c0 += kBinThreads) {
-    const long long c = c0 + t;
-    const int v = c < s.cell_cap ? __ldcg(s.cell_cnt + c) : 0;
-    int total;
-    const int ex = block_excl_scan(v, &total);
-    if (c < s.cell_cap) s.cell_start[c] = carry + ex;
-    carry += total;
-  }
-  if (t == 0) s.cell_start[s.cell_cap] = carry;
-  __syncthreads();
-  for (int i = t; i < s.nlive; i += kBinThreads) scatter_at(s, i);
-  __syncthreads();
-  for (long long c = t; c < s.cell_cap; c += kBinThreads) cellsort_at(s, cells_total, c);
-  __syncthreads();
-  for (int k = t; k < s.nlive; k += kBinThreads) stage_xs_at(s, koff, k);
+  s.xs[s.mol[m].start + k - s.cell_scan[s.grid[m].base]] = x;
 }
 
 // The lanes of a group of L lanes (L divides 32) within its warp.
@@ -418,32 +434,81 @@ __device__ __forceinline__ float slab_dist(float v, float a, float w) {
   return fmaxf(fmaxf(a - v, v - (a + w)), 0.0f);
 }
 
+// Attractive neighbour lists, a thread per bead: the bead's native row by its
+// own cut-offs, in row order (sop.cu:704-759 semantics), four entries' loads
+// in flight.  Within k_nl at 8 lanes per bead the same filter cost 19 us at
+// 50,000 beads (registers and idle lanes), as a kernel of its own 6.
+__global__ void __launch_bounds__(128) k_att(DevSys s, int koff) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.nlive) return;
+  const int m = s.mol_of[i];
+  if (!mol_listed(s, m, koff)) return;
+  if (*s.flags & FLAG_NL_OVERFLOW) return;
+  const float4* X = xbuf(s, m, koff);
+  const float4 xi = X[i];
+  const int2 row = s.nat_row[i];
+  constexpr int kB = 4;
+  int k = 0;
+  for (int e0 = 0; e0 < row.y; e0 += kB) {
+    float4 xx[kB];
+    float rc2[kB];
+#pragma unroll
+    for (int c = 0; c < kB; ++c) {
+      const int idx = row.x + min(e0 + c, row.y - 1);
+      xx[c] = X[s.nat_j[idx]];
+      rc2[c] = s.nat_rc2[idx].x;
+    }
+#pragma unroll
+    for (int c = 0; c < kB; ++c) {
+      float dx = __fsub_rn(xx[c].x, xi.x), dy = __fsub_rn(xx[c].y, xi.y),
+            dz = __fsub_rn(xx[c].z, xi.z);
+      min_image3(dx, dy, dz, s.boxl);
+      if (e0 + c < row.y && d2_exact(dx, dy, dz) < rc2[c]) s.nl_att_e[row.x + k++] = row.x + e0 + c;
+    }
+  }
+  s.nl_att_cnt[i] = k;
+}
+
 // L lanes per bead (8, or a warp for small contexts; the rows do not depend
-// on L), beads in cell order (xs), so neighbouring groups
-// share cells and candidates.  Each bead scans the cell rows (runs along x)
-// of its grid neighbourhood, culled against its own position: rows whose
-// y,z slab lies beyond the cut-off are skipped and each row's x range is
-// clipped to the chord.  Partners that pass the reference's predicate
-// (sop.cu:768-826 with the host arithmetic of sop.cu:1414-1435:
-// d^2 < (fac*sigma or abs)^2 in FP32, |i - j| > 2, not a native contact) are
-// written to the bead's fixed-stride row in candidate order (group ballot).
-// The culling is conservative (a 1e-3 A margin); membership is decided by the
-// exact predicate alone.  The bead's native partners sit in registers.
+// on L), beads in cell order (xs), so neighbouring groups share cells and
+// candidates.  Each bead scans the cell rows (runs along x) of its grid
+// neighbourhood, culled against its own position: rows whose y,z slab lies
+// beyond the cut-off are skipped and each row's x range is clipped to the
+// chord.  Partners that pass the reference's predicate (sop.cu:768-826 with the
+// host arithmetic of sop.cu:1414-1435: d^2 < (fac*sigma or abs)^2 in FP32,
+// |i - j| > 2, not a native contact) are written to the bead's fixed-stride row
+// in candidate order (group ballot).  The culling is conservative (a 1e-3 A
+// margin); membership is decided by the exact predicate alone.  The bead's
+// native partners sit in registers.
+//
+// A warp per bead (L = 32): every lane takes one cell row's bounds, and the rows'
+// candidates then form one list that the lanes walk 32 at a time (the row of
+// a candidate found by a search over the rows' prefix sums): one row after
+// another, the two dependent reads of a row's cells and three idle lanes in
+// four made the list of 4,000 beads 25.6 us (20.5 this way, the attractive
+// list included).  At 8 lanes per bead the rows fill the lanes and the search
+// costs more than it saves (50,000 beads: 304 us against 264), so each row is
+// walked by itself.
 constexpr int kNlThreads = 256;
 template <bool UNI, int L>
-__global__ void __launch_bounds__(kNlThreads) k_nl(DevSys s) {
+__global__ void __launch_bounds__(kNlThreads, 4) k_nl(DevSys s, int koff) {
   const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / L);
   const int lane = threadIdx.x % L;
   const unsigned wl = threadIdx.x & 31;
   const unsigned gmask = group_mask<L>((int)wl);
   const unsigned below = (1u << wl) - 1u;
-  if (k >= s.cell_start[s.cell_cap]) return;   // beads that were binned
-  if (*s.flags & FLAG_NL_OVERFLOW) return;
-  const float4 xi = s.xs[k];
+  if (k >= s.nlive) return;
+  const int m = s.mol_of[k];  // a molecule's staged beads lie in its own bead range
+  const float4 xi = s.xs[k];  // (stale unless the molecule was binned)
+  const bool frozen = *s.flags & FLAG_NL_OVERFLOW;
+  if (!mol_listed(s, m, koff) || frozen) return;
   const int wi = __float_as_int(xi.w);
   const int i = wi >> 2, ti = wi & 3;
-  const int m = s.mol_of[i];
+  const int mstart = s.mol[m].start;
   const MolGrid g = s.grid[m];
+  const bool chain = s.mol[m].n > kBinMolBeads;
+  const int* __restrict__ cells = chain ? s.cell_scan : s.cell_start;
+  const int shift = chain ? mstart - s.cell_scan[g.base] : 0;
   const int lc = s.bead_cell[i] - g.base;
   const int nx = g.dims[0], ny = g.dims[1], nz = g.dims[2];
   const int cx = lc % nx, cy = (lc / nx) % ny, cz = lc / (nx * ny);
@@ -457,60 +522,117 @@ __global__ void __launch_bounds__(kNlThreads) k_nl(DevSys s) {
   const float rcm = s.rc_nl_rep_max * 1.0001f + 1.0e-3f;
   const float rcm2 = rcm * rcm;
   const int2 nrow = s.nat_row[i];
+
+  if (L == 32) {
+    // attractive neighbour list: the bead's native row by its own cut-offs, in
+    // row order (sop.cu:704-759 semantics); k_att has it for L = 8
+    const float4* X = xbuf(s, m, koff);
+    int katt = 0;
+    for (int e0 = 0; e0 < nrow.y; e0 += L) {
+      const int e = e0 + lane;
+      bool pass = false;
+      if (e < nrow.y) {
+        const float4 xj = X[s.nat_j[nrow.x + e]];
+        float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y), dz = __fsub_rn(xj.z, xi.z);
+        min_image3(dx, dy, dz, boxl);
+        pass = d2_exact(dx, dy, dz) < s.nat_rc2[nrow.x + e].x;
+      }
+      const unsigned msk = __ballot_sync(gmask, pass);
+      if (pass) s.nl_att_e[nrow.x + katt + __popc(msk & below)] = nrow.x + e;
+      katt += __popc(msk);
+    }
+    if (lane == 0) s.nl_att_cnt[i] = katt;
+  }
   int nat[kNatRegs];
 #pragma unroll
   for (int q = 0; q < kNatRegs; ++q) nat[q] = q < nrow.y ? s.nat_j[nrow.x + q] : -1;
   const long long stride = s.nl_stride;
   unsigned short* row = s.nl_j + (long long)i * stride;  // partners relative to the molecule start
-  const int mstart = s.mol[m].start;
   int cnt = 0;
-  for (int z = z0; z <= z1; ++z) {
-    const float dz = g.brute ? 0.0f : slab_dist(xi.z, g.lo[2] + z * g.cs, g.cs);
-    if (dz * dz > rcm2) continue;
-    for (int y = y0; y <= y1; ++y) {
-      const float dy = g.brute ? 0.0f : slab_dist(xi.y, g.lo[1] + y * g.cs, g.cs);
-      const float rem = rcm2 - dz * dz - dy * dy;
-      if (rem < 0.0f) continue;
-      int xa = x0, xb = x1;
-      if (!g.brute) {
-        // the chord only bounds the candidates (the exact predicate decides):
-        // an approximate root and reciprocal, widened by 1e-3 A, keep it a
-        // superset at a fraction of the cost of the exact operations
-        const float w = __fmul_rn(rem, rsqrtf(fmaxf(rem, 1.0e-30f))) * 1.0001f + 1.0e-3f;
-        xa = max(x0, cell_coord_fast(xi.x - w, g.lo[0], inv_cs, nx));
-        xb = min(x1, cell_coord_fast(xi.x + w, g.lo[0], inv_cs, nx));
-      }
-      const int rowc = g.base + (z * ny + y) * nx;
-      const int ja = s.cell_start[rowc + xa];
-      const int jb = s.cell_start[rowc + xb] + s.cell_cnt[rowc + xb];
-      for (int jc = ja; jc < jb; jc += L) {
-        const int jj = jc + lane;
-        bool pass = false;
-        int j = 0;
-        if (jj < jb) {
-          const float4 xj = s.xs[jj];
-          const int wj = __float_as_int(xj.w);
-          j = wj >> 2;
-          if (abs(j - i) > 2) {
-            float dx = __fsub_rn(xj.x, xi.x), dy2 = __fsub_rn(xj.y, xi.y),
-                  dz2 = __fsub_rn(xj.z, xi.z);
-            if (wrap) min_image3(dx, dy2, dz2, boxl);
-            pass = d2_exact(dx, dy2, dz2) < (UNI ? r11 : pick_type_pair(r11, r12, r22, ti, wj & 3));
-            if (pass) {
-              bool native = false;
-#pragma unroll
-              for (int q = 0; q < kNatRegs; ++q) native |= (nat[q] == j);
-              for (int q = kNatRegs; q < nrow.y && !native; ++q) native = (s.nat_j[nrow.x + q] == j);
-              pass = !native;
-            }
-          }
-        }
-        const unsigned msk = __ballot_sync(gmask, pass);
+  // tests candidate xs[jj] and appends it to the row
+  auto candidate = [&](int jj, bool valid) {
+    bool pass = false;
+    int j = 0;
+    if (valid) {
+      const float4 xj = s.xs[jj];
+      const int wj = __float_as_int(xj.w);
+      j = wj >> 2;
+      if (abs(j - i) > 2) {
+        float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y), dz = __fsub_rn(xj.z, xi.z);
+        if (wrap) min_image3(dx, dy, dz, boxl);
+        pass = d2_exact(dx, dy, dz) < (UNI ? r11 : pick_type_pair(r11, r12, r22, ti, wj & 3));
         if (pass) {
-          const int pos = cnt + __popc(msk & below);
-          if (pos < stride) row[pos] = (unsigned short)(j - mstart);
+          bool native = false;
+#pragma unroll
+          for (int q = 0; q < kNatRegs; ++q) native |= (nat[q] == j);
+          for (int q = kNatRegs; q < nrow.y && !native; ++q) native = (s.nat_j[nrow.x + q] == j);
+          pass = !native;
         }
-        cnt += __popc(msk);
+      }
+    }
+    const unsigned msk = __ballot_sync(gmask, pass);
+    if (pass) {
+      const int pos = cnt + __popc(msk & below);
+      if (pos < stride) row[pos] = (unsigned short)(j - mstart);
+    }
+    cnt += __popc(msk);
+  };
+  // the candidates of cell row (z, y) at squared distance rcm2 - rem: xs[ja .. jb)
+  auto row_range = [&](int z, int y, float rem, int& ja, int& jb) {
+    int xa = x0, xb = x1;
+    if (!g.brute) {
+      // the chord only bounds the candidates (the exact predicate decides):
+      // an approximate root and reciprocal, widened by 1e-3 A, keep it a
+      // superset at a fraction of the cost of the exact operations
+      const float w = __fmul_rn(rem, rsqrtf(fmaxf(rem, 1.0e-30f))) * 1.0001f + 1.0e-3f;
+      xa = max(x0, cell_coord_fast(xi.x - w, g.lo[0], inv_cs, nx));
+      xb = min(x1, cell_coord_fast(xi.x + w, g.lo[0], inv_cs, nx));
+    }
+    const int rowc = g.base + (z * ny + y) * nx;
+    ja = cells[rowc + xa] + shift;
+    jb = cells[rowc + xb + 1] + shift;
+  };
+  if (L < 32) {
+    for (int z = z0; z <= z1; ++z) {
+      const float dz = g.brute ? 0.0f : slab_dist(xi.z, g.lo[2] + z * g.cs, g.cs);
+      if (dz * dz > rcm2) continue;
+      for (int y = y0; y <= y1; ++y) {
+        const float dy = g.brute ? 0.0f : slab_dist(xi.y, g.lo[1] + y * g.cs, g.cs);
+        const float rem = rcm2 - dz * dz - dy * dy;
+        if (rem < 0.0f) continue;
+        int ja, jb;
+        row_range(z, y, rem, ja, jb);
+        for (int jc = ja; jc < jb; jc += L) candidate(jc + lane, jc + lane < jb);
+      }
+    }
+  } else {
+    const int ysize = y1 - y0 + 1, nrows = (z1 - z0 + 1) * ysize;
+    for (int r0 = 0; r0 < nrows; r0 += L) {
+      int ja = 0, jb = 0;  // of row r0 + lane
+      const int r = r0 + lane;
+      if (r < nrows) {
+        const int z = z0 + r / ysize, y = y0 + r % ysize;
+        const float dz = g.brute ? 0.0f : slab_dist(xi.z, g.lo[2] + z * g.cs, g.cs);
+        const float dy = g.brute ? 0.0f : slab_dist(xi.y, g.lo[1] + y * g.cs, g.cs);
+        const float rem = rcm2 - dz * dz - dy * dy;
+        if (rem >= 0.0f) row_range(z, y, rem, ja, jb);
+      }
+      const int len = max(jb - ja, 0);
+      int end = len;  // inclusive prefix over the rows
+#pragma unroll
+      for (int o = 1; o < L; o <<= 1) {
+        const int t = __shfl_up_sync(gmask, end, o, L);
+        if (lane >= o) end += t;
+      }
+      const int total = __shfl_sync(gmask, end, L - 1, L);
+      ja -= end - len;  // candidate t of the batch is bead ja + t of its row
+      for (int t0 = 0; t0 < total; t0 += L) {
+        const int t = t0 + lane;
+        int q = 0;  // the first row whose end lies past t
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1)
+          if (__shfl_sync(gmask, end, q + o - 1, L) <= t) q += o;
+        candidate(__shfl_sync(gmask, ja, q, L) + t, t < total);
       }
     }
   }
@@ -641,45 +763,54 @@ void launch_scan(const int* in, long long n, int* out, int* block_sums, cudaStre
 long long scan_block_sums_needed(long long n) { return cdiv(n > 0 ? n : 1, kScanTile) + 1; }
 
 struct NLScratch {
-  int* ncell;        // per molecule
   int* block_sums;
-  int* cells_total;  // one int: cells in use
+  int min_mol, max_mol;  // beads of the smallest and largest molecule the context may hold
 };
 
 // Cell binning of the molecules a rebuild at koff covers: the cell order the
 // neighbour-list build walks, and each molecule's grid flags (wrap: whether
-// the minimum image can matter), which the step and pair-list kernels read;
-// att = 1 also refreshes the attractive neighbour lists.
-static void launch_binning(const DevSys& s, const NLScratch& w, int koff, int att, cudaStream_t st) {
-  if (s.nlive <= kWideListBeads && s.cell_cap <= kBinSmallCells) {
-    k_bin_small<<<1, kBinThreads, 0, st>>>(s, w.ncell, w.cells_total, koff, att);
-    return;
+// the minimum image can matter), which the step and pair-list kernels read.
+static cudaError_t launch_binning(const DevSys& s, const NLScratch& w, int koff, cudaStream_t st) {
+  if (w.min_mol <= kBinMolBeads) {
+    const int most = w.max_mol < kBinMolBeads ? w.max_mol : kBinMolBeads;
+    const size_t sm = sizeof(int) * (3 * (size_t)most + 1);
+    // a per-kernel ceiling, always the same value (contexts never lower it under
+    // one another)
+    const cudaError_t e = cudaFuncSetAttribute(k_bin_mol, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(int) * (3 * kBinMolBeads + 1));
+    if (e != cudaSuccess) return e;
+    // molecules of up to 2,048 beads take 256 threads (several blocks per SM),
+    // larger ones 1,024
+    const int threads = most <= 2048 ? 256 : 1024;
+    k_bin_mol<<<s.nmol < 2048 ? s.nmol : 2048, threads, sm, st>>>(s, koff, most);
   }
+  if (w.max_mol <= kBinMolBeads) return cudaSuccess;
   const int T = 256;
   k_bbox_reset<<<cdiv(s.nmol, T), T, 0, st>>>(s);
   k_bbox<<<cdiv(s.nlive, T), T, 0, st>>>(s, koff);
-  k_grid<<<cdiv(s.nmol, T), T, 0, st>>>(s, w.ncell, koff);
-  k_grid_base<<<1, 1024, 0, st>>>(s, w.ncell, w.cells_total);
+  k_grid<<<cdiv(s.nmol, T), T, 0, st>>>(s, koff);
   cudaMemsetAsync(s.cell_cnt, 0, sizeof(int) * (size_t)s.cell_cap, st);
-  k_assign<<<cdiv(s.nlive, T), T, 0, st>>>(s, koff, att);
-  launch_scan(s.cell_cnt, s.cell_cap, s.cell_start, w.block_sums, st);
-  k_scatter<<<cdiv(s.nlive, T), T, 0, st>>>(s);
-  k_cellsort<<<cdiv(s.cell_cap, T), T, 0, st>>>(s, w.cells_total);
+  k_assign<<<cdiv(s.nlive, T), T, 0, st>>>(s, koff);
+  launch_scan(s.cell_cnt, s.cell_cap, s.cell_scan, w.block_sums, st);
+  k_scatter<<<cdiv(s.nlive, T), T, 0, st>>>(s, koff);
+  k_cellsort<<<cdiv(s.cell_cap, T), T, 0, st>>>(s);
   k_stage_xs<<<cdiv(s.nlive, T), T, 0, st>>>(s, koff);
+  return cudaSuccess;
 }
 
 // Full neighbour-list rebuild from the coordinates at step mol_step + koff.
 void launch_nl_rebuild(const DevSys& s, const NLScratch& w, int koff, cudaStream_t st) {
   const int T = kNlThreads;
-  launch_binning(s, w, koff, 1, st);
+  launch_binning(s, w, koff, st);
   const bool wide = s.nlive <= kWideListBeads;
   const unsigned grid = cdiv((long long)s.nlive * (wide ? 32 : 8), T);
+  if (!wide) k_att<<<cdiv(s.nlive, 128), 128, 0, st>>>(s, koff);
   if (s.uniform_type) {
-    if (wide) k_nl<true, 32><<<grid, T, 0, st>>>(s);
-    else k_nl<true, 8><<<grid, T, 0, st>>>(s);
+    if (wide) k_nl<true, 32><<<grid, T, 0, st>>>(s, koff);
+    else k_nl<true, 8><<<grid, T, 0, st>>>(s, koff);
   } else {
-    if (wide) k_nl<false, 32><<<grid, T, 0, st>>>(s);
-    else k_nl<false, 8><<<grid, T, 0, st>>>(s);
+    if (wide) k_nl<false, 32><<<grid, T, 0, st>>>(s, koff);
+    else k_nl<false, 8><<<grid, T, 0, st>>>(s, koff);
   }
 }
 
@@ -688,7 +819,7 @@ void launch_nl_rebuild(const DevSys& s, const NLScratch& w, int koff, cudaStream
 // coordinates, which the step and pair-list kernels need.  The cell order
 // itself decides no result.
 void launch_rebin(const DevSys& s, const NLScratch& w, cudaStream_t st) {
-  launch_binning(s, w, 0, 0, st);
+  launch_binning(s, w, 0, st);
 }
 
 void launch_pl_rebuild(const DevSys& s, int koff, cudaStream_t st) {

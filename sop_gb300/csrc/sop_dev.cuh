@@ -32,6 +32,10 @@ namespace sop {
 
 constexpr int kMaxLanes = 32;
 
+// Molecules of up to this many beads are binned by one block each (12 bytes
+// of shared memory a bead); larger ones by a chain of kernels.
+constexpr int kBinMolBeads = 8192;
+
 // Per-molecule constants (written by the host at commit / admission).
 struct MolConst {
   int start, n;                 // bead range
@@ -49,7 +53,7 @@ struct MolGrid {
   float cs;                     // cell edge, A
   int dims[3];
   int S;                        // cells scanned on each side along each axis
-  int base;                     // first global cell index
+  int base;                     // first cell
   int ncell;
   int brute;                    // 1: index-chunked cells, all pairs scanned
   int wrap;                     // 0: no pair of the molecule can reach boxl/4 (no minimum image)
@@ -105,7 +109,9 @@ struct DevSys {
   // neighbour-list build scratch
   unsigned* bbox;               // 6 per molecule, order-preserving float bits
   MolGrid* grid;
-  int* cell_cnt; int* cell_start; long long cell_cap;
+  int* cell_start;              // first staged bead of each cell (molecules binned by one block)
+  int* cell_cnt; int* cell_scan;  // counts and their scan (larger molecules)
+  long long cell_cap;
   int* bead_cell; int* bead_slot; int* sorted; float4* xs;
   int* flags;                   // bit 0: neighbour-list overflow
   float4* noise;                // injected normals or nullptr
