@@ -21,12 +21,9 @@
 #include <algorithm>
 
 #include "reduce_dev.cuh"
-#include "sop_dev.cuh"
-#include "../../include/sop_gpu.h"
+#include "step_dev.cuh"
 
 namespace sop {
-
-constexpr int kV = 16;  // virtual lanes of the fixed force-summation order
 
 constexpr int kStepThreads = 128;  // small blocks: a finished block frees its SM slot sooner
 
@@ -36,69 +33,8 @@ struct StepBlocks {
   static constexpr int value = G == 4 ? 10 : (G == 8 ? 12 : (G == 16 ? 8 : 2));
 };
 
-// Every rounding of the per-entry arithmetic and of the accumulation is
-// written out (one rounding per operation), so the compiler cannot contract
-// it differently in different instantiations: the sums are then the same
-// bits for every lane-group width.
-__device__ __forceinline__ void acc3(float& ax, float& ay, float& az, float c, float dx, float dy,
-                                     float dz) {
-  ax = __fmaf_rn(c, dx, ax);
-  ay = __fmaf_rn(c, dy, ay);
-  az = __fmaf_rn(c, dz, az);
-}
-
-__device__ __forceinline__ float d2_plain(float dx, float dy, float dz) {
-  return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-}
-
-// Force coefficient of one bonded / angle / native entry (type 0 / 1 / 2):
-// the reference kernels' formulas, with the compensated d^2 - r0^2 wherever
-// a difference from the native distance enters.
-__device__ __forceinline__ float small_coeff(const DevSys& s, int type, float dx, float dy, float dz,
-                                             float lx, float ly, float lz, float r0, float eps,
-                                             bool& fene_bad) {
-  const float d2 = d2_plain(dx, dy, dz);
-  if (type == 0) {
-    // FENE: force on i = +k dev / (r (1 - dev^2/R0^2)) * d  (energy.cu:252-271);
-    // dev carries the compensated d^2 - r0^2, so approximate reciprocals
-    // (a few ulps) keep the term well inside the force tolerance
-    const float r = __fmul_rn(d2, rsqrtf(d2));
-    const float dev = __fmul_rn(d2_minus_r02(dx, dy, dz, lx, ly, lz, r0),
-                                __fdividef(1.0f, __fadd_rn(r, r0)));
-    const float w = __fsub_rn(1.0f, __fmul_rn(__fmul_rn(dev, dev), s.inv_R0sq));
-    fene_bad |= !(fabsf(dev) < s.R0);
-    return __fmul_rn(__fmul_rn(s.k_bnd, dev), __fdividef(1.0f, __fmul_rn(r, w)));
-  }
-  if (type == 1) {
-    // i,i+2 soft sphere: force on i = -6 eps sigma^6 / d^8 * d  (energy.cu:335-360)
-    const float inv = __fdividef(1.0f, d2);
-    const float inv2 = __fmul_rn(inv, inv);
-    return __fmul_rn(-s.f_ss, __fmul_rn(inv2, inv2));
-  }
-  // native LJ 12-6 (energy.cu:468-507): co1 = -12 eps / d^2 (s^6 - s^3),
-  // s = r0^2 / d^2, as -12 eps / d^2 s^3 (s - 1)(s^2 + s + 1) with
-  // s - 1 = -(d^2 - r0^2) / d^2; pairs with d^2 <= 1e-7 r0^2 are skipped.
-  const float r02 = __fmul_rn(r0, r0);
-  const float inv = __fdividef(1.0f, d2);
-  const float sr = __fmul_rn(r02, inv);
-  const float sm1 = __fmul_rn(-d2_minus_r02(dx, dy, dz, lx, ly, lz, r0), inv);
-  const float s3 = __fmul_rn(__fmul_rn(sr, sr), sr);
-  const float poly = __fadd_rn(__fadd_rn(__fmul_rn(sr, sr), sr), 1.0f);
-  const float c =
-      __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(-12.0f, eps), inv), __fmul_rn(s3, sm1)), poly);
-  return d2 > __fmul_rn(1.0e-7f, r02) ? c : 0.0f;
-}
-
 // STEP = false: force evaluation only at step mol_step + koff (velocities kept),
 // followed by the look-ahead; used after set-up and state uploads.
-// Marker bits in the w of a bead's force sum (0: not summed this step).
-constexpr int kSummed = 1;
-constexpr int kFeneBad = 2;   // a bond at or past R0
-constexpr int kOddStep = 4;   // the step is odd: coordinates in buffer 1
-
-template <bool STEP>
-__device__ __forceinline__ void finish_bead(const DevSys& s, int b, int m, float4 fs, int koff);
-
 // Coordinate sources of the force sum: the molecule's coordinate buffer in
 // global memory, or the block's window of it staged in shared memory (bead j
 // at xw[j - off]).  The arithmetic is the same either way, so are the bits.
@@ -121,8 +57,8 @@ struct WindowX {
 // ...).  Each physical lane holds kC = kV / G virtual lanes and does the
 // upper tree levels locally, the rest by shuffles.  So every G gives
 // bit-identical forces, and G is free to tune per context.
-template <int G, bool UNI, class XS>
-__device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, int lane,
+template <int G, bool UNI, bool wrap, class XS>
+__device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i, int m1, int lane,
                                            int2 br, int2 ar, int abase, int acnt, int rcnt,
                                            float& fx, float& fy, float& fz, bool& fene_bad) {
   constexpr int kC = kV / G;
@@ -133,10 +69,6 @@ __device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, 
                                    : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
   const float4 xi = X(i);
   const float boxl = s.boxl;
-  // 0 when no pair of the molecule can reach boxl/4 (from its last binning,
-  // with a cut-off of margin): the minimum image is then the identity and
-  // its test is skipped
-  const bool wrap = s.grid[m1].wrap != 0;
   const long long rbase = (long long)i * s.nl_stride;
 
   // Bonded, angle and native terms share one index space [bonds | angles |
@@ -174,16 +106,8 @@ __device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, 
     }
   }
 
-  // Non-native repulsion (energy.cu:536-581): co1 = -6 eps / d^2 (2 (s/r)^12 +
-  // (s/r)^6) [rep6: -6 eps / d^2 (s/r)^6]; pairs with d^2 <= 1e-7 sigma are
-  // skipped.  kC loads in flight per lane per chunk of kV entries.  A system
-  // of one bead type (UNI) uses its sigma as a constant.
-  const int ti = type_of(xi);
-  const float g11 = s.sig2[1][1], g12 = s.sig2[1][2], g22 = s.sig2[2][2];
-  const float t11 = s.rep_tol[1][1], t12 = s.rep_tol[1][2], t22 = s.rep_tol[2][2];
-  const float ce = -6.0f * s.eps_rep;
-  const float two = s.rep6 ? 0.0f : 2.0f;
-  const float q4 = 0.25f * boxl;
+  // Non-native repulsion, kC loads in flight per lane per chunk of kV entries
+  const RepConst rc = rep_const(s);
   // pair-list partners are stored relative to the molecule's first bead
   const unsigned short* __restrict__ prow = s.pl_j + rbase;
   const int jbase = s.mol[m1].start;
@@ -201,23 +125,7 @@ __device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, 
     for (int c = 0; c < kC; ++c) {
       // past the row end xx[c] is bead i itself: d2 = 0 fails the tolerance
       // test and contributes exactly 0, so no branch is needed
-      float dx = __fsub_rn(xx[c].x, xi.x), dy = __fsub_rn(xx[c].y, xi.y),
-            dz = __fsub_rn(xx[c].z, xi.z);
-      // |dx| + |dy| + |dz| bounds every component: one test for the rare wrap
-      if (wrap && fabsf(dx) + fabsf(dy) + fabsf(dz) > q4) min_image3(dx, dy, dz, boxl);
-      const float d2 = d2_plain(dx, dy, dz);
-      float sg2 = g11, tol = t11;
-      if (!UNI) {
-        const int tj = type_of(xx[c]);
-        sg2 = pick_type_pair(g11, g12, g22, ti, tj);
-        tol = pick_type_pair(t11, t12, t22, ti, tj);
-      }
-      const float inv = __fdividef(1.0f, d2);
-      const float u = __fmul_rn(sg2, inv);
-      const float u3 = __fmul_rn(__fmul_rn(u, u), u);
-      const float cc = (d2 > tol) ? __fmul_rn(__fmul_rn(__fmul_rn(ce, inv), u3), __fmaf_rn(two, u3, 1.0f))
-                                  : 0.0f;
-      acc3(ax[c], ay[c], az[c], cc, dx, dy, dz);
+      rep_entry<UNI, wrap>(rc, xi, xx[c], ax[c], ay[c], az[c]);
     }
   }
   // upper levels of the fixed tree inside the lane, lower levels by shuffles
@@ -242,6 +150,20 @@ __device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, 
   fx = ax[0];
   fy = ay[0];
   fz = az[0];
+}
+
+// wrap is 0 when no pair of the molecule can reach boxl/4 (from its last
+// binning, with a cut-off of margin): the minimum image is then the identity.
+// The test of every entry then costs more than its arithmetic saves branches,
+// so the sum is compiled for both.
+template <int G, bool UNI, class XS>
+__device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, int lane,
+                                           int2 br, int2 ar, int abase, int acnt, int rcnt,
+                                           float& fx, float& fy, float& fz, bool& fene_bad) {
+  if (s.grid[m1].wrap)
+    bead_force_w<G, UNI, true>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
+  else
+    bead_force_w<G, UNI, false>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
 }
 
 // SPLIT = false: one kernel -- the groups' sums go through shared memory to
@@ -293,15 +215,6 @@ __device__ __forceinline__ BeadSlot bead_slot(const DevSys& s, int b1, int koff)
       q.i = b1;
   }
   return q;
-}
-
-// The force sum's w: the marker bits of finish_bead (summed, a bond past R0,
-// the parity of the step, which selects the coordinate buffers).
-__device__ __forceinline__ float4 marked_sum(float fx, float fy, float fz, bool fene_bad,
-                                             long long n) {
-  return make_float4(fx, fy, fz,
-                     __int_as_float(kSummed | (fene_bad ? kFeneBad : 0) |
-                                    ((int)(n & 1) ? kOddStep : 0)));
 }
 
 template <int G, bool STEP, bool UNI, bool SPLIT, bool WIN>
@@ -372,86 +285,6 @@ __global__ void __launch_bounds__(kStepThreads, StepBlocks<G>::value) k_step(Dev
   const int b = bead[threadIdx.x];
   if (b < 0) return;
   finish_bead<STEP>(s, b, s.mol_of[b], fsum[threadIdx.x], koff);
-}
-
-// What completing bead b (of molecule m) at step mol_step + STEP + koff needs
-// besides its force sum: its state (coordinates from buffer cur, the step's
-// parity) and its noise.  None of it is written by the force kernel of the
-// same step.
-struct BeadState {
-  MolConst mc;
-  long long nb;
-  float4 vi, inc, xo, pi;
-  float3 z;
-};
-
-template <bool STEP>
-__device__ __forceinline__ void load_bead_state(const DevSys& s, int b, int m, int koff, int cur,
-                                                BeadState& t) {
-  t.mc = s.mol[m];
-  t.nb = s.mol_step[m] + (STEP ? 1 : 0) + koff;
-  t.vi = s.v[b];
-  t.inc = s.incr[b];
-  t.xo = s.x[cur][b];
-  t.pi = s.p[cur][b];
-  if (s.use_noise) {
-    const float4 q = s.noise[b];
-    t.z = make_float3(q.x, q.y, q.z);
-  } else {
-    t.z = noise3((unsigned)(b - t.mc.start), t.nb, t.mc.traj, s.seed_lo, s.seed_hi);
-  }
-}
-
-// Completes bead b from its conservative force sum fs, whose w holds the
-// marker bits k_step set: noise, status, velocity and the look-ahead
-// position update (sop.cu:421-462, energy.cu:588-604).  Every rounding is
-// written out.
-template <bool STEP>
-__device__ __forceinline__ void complete_bead(const DevSys& s, int b, int m, float4 fs, int cur,
-                                              const BeadState& t) {
-  const int w = __float_as_int(fs.w);
-  const MolConst& mc = t.mc;
-  float4 vi = t.vi;
-  float4 inc = t.inc;
-  const float4 xo = t.xo;
-  const float4 pi = t.pi;
-  const float3 z = t.z;
-  const float fxx = __fmaf_rn(mc.sigma_f, z.x, fs.x);
-  const float fyy = __fmaf_rn(mc.sigma_f, z.y, fs.y);
-  const float fzz = __fmaf_rn(mc.sigma_f, z.z, fs.z);
-  int st = 0;
-  if (w & kFeneBad) st |= SOP_MOL_FENE_RANGE;
-  if (!(isfinite(fxx) && isfinite(fyy) && isfinite(fzz))) st |= SOP_MOL_NONFINITE;
-  if (st) atomicOr(s.mol_status + m, st);
-  s.f[b] = make_float4(fxx, fyy, fzz, 0.f);
-  // step 0 is the initial force evaluation (sop.cu:180-186): velocities stay
-  if (STEP && t.nb > 0 && !mc.t_zero) {
-    vi = make_float4(__fmaf_rn(mc.a3, inc.x, __fmul_rn(mc.a4, fxx)),
-                     __fmaf_rn(mc.a3, inc.y, __fmul_rn(mc.a4, fyy)),
-                     __fmaf_rn(mc.a3, inc.z, __fmul_rn(mc.a4, fzz)), 0.f);
-    s.v[b] = vi;
-  }
-  inc = make_float4(__fmaf_rn(mc.a1, vi.x, __fmul_rn(mc.a2, fxx)),
-                    __fmaf_rn(mc.a1, vi.y, __fmul_rn(mc.a2, fyy)),
-                    __fmaf_rn(mc.a1, vi.z, __fmul_rn(mc.a2, fzz)), 0.f);
-  s.incr[b] = inc;
-  s.x[cur ^ 1][b] = make_float4(__fadd_rn(xo.x, inc.x), __fadd_rn(xo.y, inc.y),
-                                __fadd_rn(xo.z, inc.z), xo.w);
-  const float boxl = s.boxl;
-  s.p[cur ^ 1][b] = make_float4(min_image(__fadd_rn(pi.x, inc.x), boxl),
-                                min_image(__fadd_rn(pi.y, inc.y), boxl),
-                                min_image(__fadd_rn(pi.z, inc.z), boxl), 0.f);
-}
-
-// Completes bead b (of molecule m) from its force sum fs; the step is the
-// molecule's mol_step + STEP + koff, as in k_step, and its parity (which
-// selects the coordinate buffers) is marked in fs.w.
-template <bool STEP>
-__device__ __forceinline__ void finish_bead(const DevSys& s, int b, int m, float4 fs, int koff) {
-  const int cur = (__float_as_int(fs.w) & kOddStep) ? 1 : 0;
-  BeadState t;
-  load_bead_state<STEP>(s, b, m, koff, cur, t);
-  complete_bead<STEP>(s, b, m, fs, cur, t);
 }
 
 // Second kernel of the split step: completes every bead k_step summed
