@@ -184,12 +184,15 @@ def whole_job_rate(beads_per_rank: int, md_steps: int, world: int, t_max: float)
     return world * beads_per_rank * md_steps / t_max
 
 
-def launches_per_bench_step(p, s0: int, form: int = 1, beads: int = 0, largest: int = 0) -> int:
+def launches_per_bench_step(p, s0: int, form: int = 1, beads: int = 0, smallest: int = 0,
+                            largest: int = 0) -> int:
     """Kernels of the engine in one replay starting after step s0 (form 1:
     one step kernel per step; 2: force + finish kernels; 3 and 4: one
     launch per run of steps between list rebuilds), in a context of `beads`
-    beads whose largest molecule has `largest`."""
-    nl_kernels = 2     # bin_mol, nl
+    beads whose molecules have `smallest` to `largest`."""
+    nl_kernels = 1     # nl
+    if smallest <= 8192:
+        nl_kernels += 1    # bin_mol
     if beads > 16384:
         nl_kernels += 1    # att
     if largest > 8192:
@@ -425,7 +428,8 @@ def plain_measure(workload: str, local: int, K: int, warmup: int, lanes: int = 0
     tuning = e.tuning()
     e.close()
     s0 = stages[names[0]]
-    n_launch = sum(launches_per_bench_step(p, s_start + k * MD_STEPS, tuning["form"], mol.n, mol.n)
+    n_launch = sum(launches_per_bench_step(p, s_start + k * MD_STEPS, tuning["form"], mol.n, mol.n,
+                                           mol.n)
                    for k in range(K))
     cpu = None
     if cpu_seconds > 0:
@@ -733,7 +737,7 @@ def main() -> None:
 
     if rank == 0:
         n_launch = sum(launches_per_bench_step(p, s0_ + k * MD_STEPS, tu.get("form", 1), sum(ns),
-                                               max(ns))
+                                               min(ns), max(ns))
                        for s0_, tu, ns in zip(s_start, tuning, part_sizes) for k in range(K))
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K,

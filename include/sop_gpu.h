@@ -85,9 +85,11 @@ typedef struct sop_params {
                          finish kernel, 3 every step between two list rebuilds
                          in one cooperative launch (a device-wide barrier
                          between steps), 4 the same in one block of 1,024
-                         threads (block barriers; tried by the tuner for
-                         contexts of up to 2,048 bead slots), 0 chosen by
-                         timing at commit (served contexts: 2).  Every form
+                         threads (block barriers), 0 chosen at commit: form 1
+                         for plain and batched contexts of up to 16,384 bead
+                         slots (with 0 or 1, and 0, 8 or 16 lanes per bead, its
+                         reads are then staged in shared memory), by timing
+                         for larger ones (served contexts: 2).  Every form
                          gives the same bits. */
   int step_window;    /* shared-memory window of the step, in beads: each step
                          block stages the coordinates of its beads' molecules

@@ -49,6 +49,13 @@ cudaError_t launch_barrier_check(const DevSys& s, int G, unsigned* bar, int miss
 void launch_step_tiles(const DevSys& s, int koff, bool step, const int4* tiles, int ntiles,
                        bool any_split, cudaStream_t st);
 void launch_advance(const DevSys& s, int steps, cudaStream_t st);
+// kernels_tile.cu
+cudaError_t launch_step_tile(const DevSys& s, const TileSet& ts, int koff, bool early,
+                             cudaStream_t st);
+cudaError_t launch_pl_tile(const DevSys& s, const TileSet& ts, int koff, bool only_tables,
+                           cudaStream_t st);
+cudaError_t launch_pair_step(const DevSys& s, int lanes, int koff, bool early, int max_mol,
+                             cudaStream_t st);
 void launch_gather_current(const DevSys& s, float* out, int* flag_out, cudaStream_t st);
 int energy_blocks(int mol_n);
 void launch_energy(const DevSys& s, int mol_start, int mol_n, int m, double* part, double* out,
@@ -200,6 +207,8 @@ struct SopCtx {
   int wcap = 0;               // > 0: step blocks stage their molecules (up to wcap beads)
   bool persist = false;       // steps between list rebuilds in one cooperative launch
   bool one_block = false;     // steps between list rebuilds in one block
+  TileSet tiles{};            // tables of the tile step (tiles.beads 0: not used)
+  int pair_step = 0;          // lanes per bead of pair-list rebuild and step in one launch (0: apart)
   // tiled form: per-molecule tiles, lanes and form chosen per size bucket
   bool tiled = false;
   int4* d_tiles = nullptr;    // {first bead, end bead, lanes, two-kernel form}
@@ -315,6 +324,9 @@ namespace {
 
 int graph_steps(const SopCtx* ctx);
 
+// The steps run staged (kernels_tile.cu).
+bool staged(const SopCtx* ctx) { return ctx->tiles.beads || ctx->pair_step; }
+
 // The rows of the molecule whose beads are o .. o + n - 1 in the repulsive
 // neighbour list (r = 0) or pair list (r = 1), every entry as an index
 // relative to bead o (as stored), full row stride.
@@ -393,7 +405,8 @@ int autotune_lanes(SopCtx* ctx) {
     if (fixed_g && g != fixed_g) continue;
     float gbest = 1e30f;
     for (int f = 1; f <= 4; ++f) {
-      if (fixed_f ? f != fixed_f : (f == 3 || (f == 4 && ctx->s.nlive > kOneBlockMaxBeads)))
+      if (fixed_f ? f != fixed_f
+                  : (f == 3 || (f == 4 && (ctx->s.nlive > kOneBlockMaxBeads || staged(ctx)))))
         continue;
       if (f >= 3 && ctx->served) continue;
       const bool sp = f == 2;
@@ -492,6 +505,74 @@ int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol = -1) {
   return ctx->fail(SOP_ERR_CAPACITY, "neighbour list kept overflowing");
 }
 
+// Pair-list rebuild of the molecules of s, and of the tables the tile step
+// reads them from.
+void rebuild_pairs(SopCtx* ctx, const DevSys& s, int koff) {
+  if (ctx->tiles.beads) launch_pl_tile(s, ctx->tiles, koff, false, ctx->stream);
+  else launch_pl_rebuild(s, koff, ctx->stream);
+}
+
+// Copies the coordinates to where k_pair_step reads the last step's: after
+// every change of them other than by its own steps.
+int keep_last(SopCtx* ctx) {
+  if (!ctx->pair_step) return SOP_OK;
+  for (int b = 0; b < 2; ++b)
+    CK(cudaMemcpyAsync(ctx->s.xl[b], ctx->s.x[b], sizeof(float4) * (size_t)ctx->s.nbead,
+                       cudaMemcpyDeviceToDevice, ctx->stream));
+  return SOP_OK;
+}
+
+// The steps of small contexts with their reads staged in shared memory
+// (kernels_tile.cu): the one-kernel form, so they serve where that form may
+// (step_split 0 or 1, no window, no size buckets asked for, a lane count they
+// are built for).  Contexts with a pair list before every step take the rebuild
+// and the step in one launch, others tiles of `beads` beads.
+// Above kStagedBeads the kernels fill the GPU and the one-kernel form is as
+// fast without tables.  us per 50 steps staged / not, one molecule, pair list
+// every 10 steps: 2,000 beads 447 / 575, 8,000 620 / 695 (16 beads a tile),
+// 12,000 757 / 816, 16,000 875 / 999 (32), 24,000 1,272 / 1,170; before every
+// step (factor cut-offs): 128 beads 389 / 570, 2,000 529 / 686, 8,000 682 / 980,
+// 16,000 833 / 1,188.
+constexpr long long kStagedBeads = 16384, kStagedSmall = 8192;
+int alloc_staged(SopCtx* ctx) {
+  const sop_params& P = ctx->P;
+  TileSet& ts = ctx->tiles;
+  ts = TileSet{};
+  ctx->pair_step = 0;
+  const int lanes = lanes_for(ctx);
+  if (ctx->served || P.step_split > 1 || P.step_window > 0 || P.step_buckets > 0 ||
+      ctx->s.nbead > kStagedBeads)
+    return SOP_OK;
+  if (P.nplup <= 1) {
+    if (lanes && lanes != 8 && lanes != 16) return SOP_OK;
+    for (int b = 0; b < 2; ++b) {
+      ctx->s.xl[b] = ctx->dalloc<float4>(ctx->s.nbead);
+      if (!ctx->s.xl[b]) return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
+    }
+    // 8 lanes for larger contexts, but not for long rows (up to 512 entries at
+    // the factor cut-offs, 1,088 at 32 A): us per 50 steps with 8 / 16 lanes,
+    // 8,000 beads 708 / 682, 12,000 758 / 901; 10,900 beads at 32 A 1,354 / 1,096
+    const bool eight = ctx->s.nbead > kStagedSmall && ctx->s.nl_stride <= 512;
+    ctx->pair_step = lanes ? lanes : eight ? 8 : 16;
+    return keep_last(ctx);
+  }
+  if (lanes && lanes != 8 && lanes != 16) return SOP_OK;
+  const int tb = lanes ? 256 / lanes : ctx->s.nbead <= kStagedSmall ? 16 : 32;
+  const size_t n = ((size_t)ctx->s.nbead + tb - 1) / tb;
+  ts.ntile = (int)n;
+  ts.smem = kTileSmemMost;
+  ts.cnt = ctx->dalloc<int>(n);
+  ts.bead = ctx->dalloc<int>(n * kTileCap);
+  ts.dim = ctx->dalloc<int2>(n);
+  ts.num = ctx->dalloc<int>(ctx->s.nbead);
+  ts.rep = ctx->dalloc<unsigned short>(n * tb * 16 * kTileChunks);
+  ts.small = ctx->dalloc<float4>(n * tb * kTileSmall);
+  if (!ts.cnt || !ts.bead || !ts.dim || !ts.num || !ts.rep || !ts.small)
+    return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
+  ts.beads = tb;
+  return SOP_OK;
+}
+
 void force_eval_async(SopCtx* ctx) {
   launch_step(ctx->s, ctx->G, ctx->split, 0, false, ctx->wcap, ctx->stream);
 }
@@ -500,6 +581,12 @@ void force_eval_async(SopCtx* ctx) {
 // among them): one persistent launch, or one launch per step.
 void launch_steps(SopCtx* ctx, int koff0, int count) {
   if (count <= 0) return;
+  if (ctx->tiles.beads) {
+    // the first follows a rebuild or a clock advance
+    for (int k = koff0; k < koff0 + count; ++k)
+      launch_step_tile(ctx->s, ctx->tiles, k, k > koff0, ctx->stream);
+    return;
+  }
   if (ctx->tiled) {
     for (int k = koff0; k < koff0 + count; ++k)
       launch_step_tiles(ctx->s, k, true, ctx->d_tiles, ctx->ntiles, ctx->tiles_split, ctx->stream);
@@ -535,6 +622,21 @@ int rebuilds_before(const sop_params& P, long long n) {
 void enqueue_block(SopCtx* ctx, long long s0, int count) {
   int run0 = 0;  // first step of the current run without rebuilds
   int base = 0;  // steps of the block the clocks already count
+  if (ctx->pair_step) {  // the pair-list rebuild precedes every step, in its launch
+    bool early = false;  // a step is the launch before
+    for (int k = 0; k < count; ++k) {
+      if (rebuilds_before(ctx->P, s0 + 1 + k) & 1) {
+        if (k > base) launch_advance(ctx->s, k - base, ctx->stream);
+        base = k;
+        launch_nl_rebuild(ctx->s, ctx->w, 0, ctx->stream);
+        early = false;
+      }
+      launch_pair_step(ctx->s, ctx->pair_step, k - base, early, ctx->w.max_mol, ctx->stream);
+      early = true;
+    }
+    launch_advance(ctx->s, count - base, ctx->stream);
+    return;
+  }
   for (int k = 0; k < count; ++k) {
     int r = rebuilds_before(ctx->P, s0 + 1 + k);
     if (r) {
@@ -546,7 +648,7 @@ void enqueue_block(SopCtx* ctx, long long s0, int count) {
       base = k;
     }
     if (r & 1) launch_nl_rebuild(ctx->s, ctx->w, k - base, ctx->stream);
-    if (r & 2) launch_pl_rebuild(ctx->s, k - base, ctx->stream);
+    if (r & 2) rebuild_pairs(ctx, ctx->s, k - base);
   }
   launch_steps(ctx, run0 - base, count - run0);
   launch_advance(ctx->s, count - base, ctx->stream);
@@ -754,6 +856,7 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   s.sorted = ctx->dalloc<int>(nb);
   s.xs = ctx->dalloc<float4>(nb);
   s.flags = ctx->dalloc<int>(4);  // [0] flags, [2..3] the persistent step's barrier
+  s.xl[0] = s.xl[1] = nullptr;
   s.noise = nullptr;
   s.use_noise = 0;
   ctx->w.min_mol = (int)c.min_mol_beads;
@@ -1129,14 +1232,14 @@ int setup_step0(SopCtx* ctx) {
   // current step itself (x_0 sits in both coordinate buffers)
   int rc = nl_rebuild_checked(ctx, -1);
   if (rc) return rc;
-  launch_pl_rebuild(ctx->s, -1, ctx->stream);
+  rebuild_pairs(ctx, ctx->s, -1);
   force_eval_async(ctx);
   CK(cudaGetLastError());
   if (!fixed_g || !fixed_f) {
     rc = autotune_lanes(ctx);
     if (rc) return rc;
   }
-  if (!fixed_g && !fixed_f && !ctx->served) {
+  if (!fixed_g && !fixed_f && !ctx->served && !staged(ctx)) {
     rc = autotune_buckets(ctx);
     if (rc) return rc;
   } else if (ctx->P.step_buckets > 0 && !ctx->served) {
@@ -1216,6 +1319,8 @@ int commit(SopCtx* ctx) {
   }
   for (int k = 0; k < nm; ++k) ctx->mc[k] = all.mc[k];
   rc = upload_staged(ctx, all);
+  if (rc) return rc;
+  rc = alloc_staged(ctx);
   if (rc) return rc;
   rc = setup_step0(ctx);
   if (rc) return rc;
@@ -1911,7 +2016,9 @@ int sop_upload_state(void* p, int mol, const float* pos, const float* unc_pos, c
   if (rc) return rc;
   DevSys one = ctx->s;
   one.only_mol = mol;
-  launch_pl_rebuild(one, -1, ctx->stream);
+  rc = keep_last(ctx);
+  if (rc) return rc;
+  rebuild_pairs(ctx, one, -1);
   force_eval_async(ctx);  // every molecule: the same forces again for the others
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1949,8 +2056,11 @@ int sop_launch_stage(void* p, int stage, int koff) {
   SopCtx* ctx = C(p);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   switch (stage) {
-    case 0: launch_steps(ctx, koff, 1); break;
-    case 1: launch_pl_rebuild(ctx->s, koff, ctx->stream); break;
+    case 0:
+      if (ctx->pair_step) CK(launch_pair_step(ctx->s, ctx->pair_step, koff, false, ctx->w.max_mol, ctx->stream));
+      else launch_steps(ctx, koff, 1);
+      break;
+    case 1: rebuild_pairs(ctx, ctx->s, koff); break;
     case 2: launch_nl_rebuild(ctx->s, ctx->w, koff, ctx->stream); break;
     case 3: launch_advance(ctx->s, koff, ctx->stream); break;
     default: return ctx->fail(SOP_ERR_ARG, "unknown stage");
@@ -1986,7 +2096,7 @@ int sop_update_pair_list(void* p, long long* nil_att, long long* nil_rep) {
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
-  launch_pl_rebuild(ctx->s, 0, ctx->stream);
+  rebuild_pairs(ctx, ctx->s, 0);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   if (nil_att || nil_rep) {
@@ -2310,6 +2420,9 @@ int sop_restore(void* p, int mol, const void* buf, long long size) {
   // refresh each molecule's grid flags (and the cell order) from the restored
   // coordinates: binning only, no list changes
   launch_rebin(ctx->s, ctx->w, ctx->stream);
+  if (ctx->tiles.beads) CK(launch_pl_tile(ctx->s, ctx->tiles, 0, true, ctx->stream));
+  rc = keep_last(ctx);
+  if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   if (set_clock) {
@@ -2376,7 +2489,7 @@ int sop_memory(void* p, int mol, long long* ctx_bytes, long long* mol_bytes) {
 int sop_tuning(void* p, int* lanes, float* ms) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
-  if (lanes) *lanes = ctx->G;
+  if (lanes) sop_step_form(p, lanes, nullptr);
   if (ms) {
     const int cand[4] = {2, 4, 8, 16};
     for (int k = 0; k < 4; ++k) {
@@ -2390,8 +2503,8 @@ int sop_tuning(void* p, int* lanes, float* ms) {
 int sop_step_form(void* p, int* lanes, int* form) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
-  if (lanes) *lanes = ctx->G;
-  if (form) *form = ctx->one_block ? 4 : ctx->persist ? 3 : ctx->split ? 2 : 1;
+  if (lanes) *lanes = ctx->tiles.beads ? 256 / ctx->tiles.beads : ctx->pair_step ? ctx->pair_step : ctx->G;
+  if (form) *form = staged(ctx) ? 1 : ctx->one_block ? 4 : ctx->persist ? 3 : ctx->split ? 2 : 1;
   return SOP_OK;
 }
 

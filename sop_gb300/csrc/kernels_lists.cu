@@ -22,7 +22,7 @@
 //                                                                          k_nl
 // Pair list (every nplup steps): eight lanes per bead, beads in chain order,
 // compact its neighbour-list row in row order (k_pl).
-#include "sop_dev.cuh"
+#include "lists_dev.cuh"
 
 namespace sop {
 
@@ -118,23 +118,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
 // one more entry of cell_start, which 3 n hold, so the ranges of molecules are
 // apart wherever their beads are.
 __device__ __forceinline__ int cell_base(int start) { return 3 * start; }
-
-// Molecules whose lists a rebuild at block offset koff refreshes: running,
-// healthy, and with the step this rebuild precedes (mol_step + koff + 1)
-// still within the step budget -- a molecule that has finished keeps the
-// lists of its last step, as the reference's loop ends there.
-__device__ __forceinline__ bool mol_listed(const DevSys& s, int m, int koff) {
-  if (m < 0) return false;
-  if (s.only_mol >= 0 && m != s.only_mol) return false;  // its lists and grid stay
-  const MolConst& mc = s.mol[m];
-  return mc.active && s.mol_status[m] == 0 &&
-         !(mc.nsteps >= 0 && s.mol_step[m] + koff >= mc.nsteps);
-}
-
-// Coordinates at step mol_step + koff (the positions the rebuild uses).
-__device__ __forceinline__ const float4* xbuf(const DevSys& s, int m, int koff) {
-  return s.x[(int)((s.mol_step[m] + koff) & 1)];
-}
 
 __device__ __forceinline__ bool bins_by_chain(const DevSys& s, int m, int koff) {
   return mol_listed(s, m, koff) && s.mol[m].n > kBinMolBeads;
@@ -410,12 +393,6 @@ __global__ void k_stage_xs(DevSys s, int koff) {
   s.xs[s.mol[m].start + k - s.cell_scan[s.grid[m].base]] = x;
 }
 
-// The lanes of a group of L lanes (L divides 32) within its warp.
-template <int L>
-__device__ __forceinline__ unsigned group_mask(int wl) {
-  return L == 32 ? 0xffffffffu : (((1u << L) - 1u) << (wl & ~(L - 1)));
-}
-
 // Contexts of up to this many bead slots rebuild their lists with a warp
 // per bead: at 8 lanes per bead they fill less than a wave of the GPU.
 constexpr int kWideListBeads = 16384;
@@ -645,108 +622,23 @@ __global__ void __launch_bounds__(kNlThreads, 4) k_nl(DevSys s, int koff) {
   }
 }
 
-// L lanes per bead (8: four beads per warp; 16 for molecules whose rows are
-// long; 32: a warp per bead, for small contexts, where fewer than a wave of
-// beads leaves the latency of each bead's rounds exposed): the pair list is
-// the in-order compaction of the bead's neighbour-list row by the pair-list
-// cut-off (sop.cu:835-920 semantics, host arithmetic of sop.cu:1737-1810).  Each lane takes 4
-// consecutive entries per round (one 8-byte load, four independent gathers)
-// and a scan across the group places the survivors; the attractive pair
-// list is the same over the bead's attractive neighbour list.  The lists do
-// not depend on L.
+// L lanes per bead: 8 (four beads per warp), 16 for molecules whose rows are
+// long, or a warp per bead for small contexts, where fewer than a wave of
+// beads leaves the latency of each bead's rounds exposed.  Beads in chain
+// order: the groups of a block gather from the same region of a molecule,
+// and the per-bead loads are coalesced.
 template <bool UNI, int L>
 __global__ void __launch_bounds__(256, 5) k_pl(DevSys s, int koff) {  // 48 registers: 5 blocks per SM
   pdl_wait();
   pdl_release();
-  const int wl = threadIdx.x & 31;
-  const int lane = wl & (L - 1);
-  const unsigned gmask = group_mask<L>(wl);
-  // beads in chain order: the groups of a block gather from the same region
-  // of a molecule, and the per-bead loads are coalesced
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / L);
   if (i >= s.nlive) return;
   if (*s.flags & FLAG_NL_OVERFLOW) return;
   const int m = s.mol_of[i];
   if (!mol_listed(s, m, koff)) return;  // finished or stopped: keeps the lists of its last step
-  const float4* X = xbuf(s, m, koff);
-  const float4 xi = X[i];
-  const int ti = type_of(xi);
-  const float boxl = s.boxl;
-  const bool wrap = s.grid[m].wrap != 0;  // from the neighbour-list build, with a cut-off of margin
-  const float r11 = s.rc2_pl_rep[1][1], r12 = s.rc2_pl_rep[1][2], r22 = s.rc2_pl_rep[2][2];
-  const unsigned below = (1u << wl) - 1u;  // lanes of the warp before this one
-  const long long a = (long long)i * s.nl_stride;
-  // rows hold partners relative to the molecule's first bead, 4 per 8 bytes
-  const uint2* row4 = reinterpret_cast<const uint2*>(s.nl_j + a);
-  unsigned short* out = s.pl_j + a;
-  const int mstart = s.mol[m].start;
-  const unsigned irel = (unsigned)(i - mstart);
-  const unsigned self2 = irel | (irel << 16);  // two entries that name bead i
-  const int cnt = s.nl_cnt[i];
-  const int2 row = s.nat_row[i];
-  const int acnt = s.nl_att_cnt[i];
-  int k = 0;
-  // each round works on entries loaded the round before (rows are read ahead)
-  uint2 jn = make_uint2(self2, self2);
-  if (4 * lane < cnt) jn = row4[lane];
-  for (int e0 = 0; e0 < cnt; e0 += 4 * L) {
-    const int e = e0 + 4 * lane;
-    const uint2 jv = jn;
-    jn = make_uint2(self2, self2);
-    if (e + 4 * L < cnt) jn = row4[(e0 >> 2) + L + lane];
-    const int jq[4] = {mstart + (int)(jv.x & 0xffffu),
-                       e + 1 < cnt ? mstart + (int)(jv.x >> 16) : i,
-                       e + 2 < cnt ? mstart + (int)(jv.y & 0xffffu) : i,
-                       e + 3 < cnt ? mstart + (int)(jv.y >> 16) : i};
-    unsigned pb = 0;
-    int c = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 xj = X[jq[q]];
-      float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y),
-            dz = __fsub_rn(xj.z, xi.z);
-      if (wrap) min_image3(dx, dy, dz, boxl);
-      const bool p = (e + q < cnt) &&
-                     d2_exact(dx, dy, dz) < (UNI ? r11 : pick_type_pair(r11, r12, r22, ti, type_of(xj)));
-      pb |= (p ? 1u : 0u) << q;
-      c += p ? 1 : 0;
-    }
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) {
-      const int t = __shfl_up_sync(gmask, incl, o, L);
-      if (lane >= o) incl += t;
-    }
-    int pos = k + incl - c;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (pb & (1u << q)) out[pos++] = (unsigned short)(jq[q] - mstart);
-    k += __shfl_sync(gmask, incl, L - 1, L);
-  }
-  if (lane == 0) s.pl_cnt[i] = k;
-  int ka = 0;
-  for (int e0 = 0; e0 < acnt; e0 += L) {
-    const int e = e0 + lane;
-    bool pass = false;
-    int j = 0;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (e < acnt) {
-      const int idx = s.nl_att_e[row.x + e];
-      // the contact's partner, cut-off and parameters in one round of loads
-      j = s.nat_j[idx];
-      const float rc2 = s.nat_rc2[idx].y;
-      q = s.nat_par[idx];
-      const float4 xj = X[j];
-      float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y),
-            dz = __fsub_rn(xj.z, xi.z);
-      if (wrap) min_image3(dx, dy, dz, boxl);
-      pass = d2_exact(dx, dy, dz) < rc2;
-    }
-    const unsigned mask = __ballot_sync(gmask, pass) & gmask;
-    if (pass) s.pl_att[row.x + ka + __popc(mask & below)] = make_float4(__int_as_float(j), q.x, q.y, q.z);
-    ka += __popc(mask);
-  }
-  if (lane == 0) s.pl_att_cnt[i] = ka;
+  int nrep, natt;
+  pair_rows<UNI, L>(
+      s, xbuf(s, m, koff), i, pair_head<L>(s, i, m), [](int, int) {}, [](int, float4) {}, nrep, natt);
 }
 
 // ------------------------------------------------------------ host side

@@ -21,7 +21,7 @@
 #include <algorithm>
 
 #include "reduce_dev.cuh"
-#include "step_dev.cuh"
+#include "step_force.cuh"
 
 namespace sop {
 
@@ -35,137 +35,6 @@ struct StepBlocks {
 
 // STEP = false: force evaluation only at step mol_step + koff (velocities kept),
 // followed by the look-ahead; used after set-up and state uploads.
-// Coordinate sources of the force sum: the molecule's coordinate buffer in
-// global memory, or the block's window of it staged in shared memory (bead j
-// at xw[j - off]).  The arithmetic is the same either way, so are the bits.
-struct GlobalX {
-  const float4* __restrict__ p;
-  __device__ __forceinline__ float4 operator()(int j) const { return p[j]; }
-};
-struct WindowX {
-  const float4* p;  // shared memory
-  int off;
-  __device__ __forceinline__ float4 operator()(int j) const { return p[j - off]; }
-};
-
-// The conservative force on bead i, summed by the G lanes of its group over
-// its rows (bonds, angles, native pair list, repulsive pair list) into the
-// lane's kC virtual-lane accumulators, reduced to lane 0 of the group.
-// Forces are summed in a fixed order whatever G is: entry e of a row
-// accumulates into virtual lane e % kV (in increasing e), and the kV partial
-// sums combine in one fixed binary tree (pairs v, v + kV/2, then v, v + kV/4,
-// ...).  Each physical lane holds kC = kV / G virtual lanes and does the
-// upper tree levels locally, the rest by shuffles.  So every G gives
-// bit-identical forces, and G is free to tune per context.
-template <int G, bool UNI, bool wrap, class XS>
-__device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i, int m1, int lane,
-                                           int2 br, int2 ar, int abase, int acnt, int rcnt,
-                                           float& fx, float& fy, float& fz, bool& fene_bad) {
-  constexpr int kC = kV / G;
-  float ax[kC], ay[kC], az[kC];
-#pragma unroll
-  for (int c = 0; c < kC; ++c) ax[c] = ay[c] = az[c] = 0.f;
-  const unsigned gmask = (G == 32) ? 0xffffffffu
-                                   : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-  const float4 xi = X(i);
-  const float boxl = s.boxl;
-  const long long rbase = (long long)i * s.nl_stride;
-
-  // Bonded, angle and native terms share one index space [bonds | angles |
-  // natives]; a bead has a handful of them, usually one pass.
-  const int nba = br.y + ar.y;
-  const int nsmall = nba + acnt;
-  for (int base = 0; base < nsmall; base += kV) {
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      const int e = base + lane + c * G;
-      if (e >= nsmall) continue;
-      int j, t;
-      float r0 = 0.f, eps = 0.f;
-      if (e < br.y) {
-        j = s.bond_j[br.x + e];
-        r0 = s.bond_r0[br.x + e];
-        t = 0;
-      } else if (e < nba) {
-        j = s.ang_j[ar.x + e - br.y];
-        t = 1;
-      } else {
-        const float4 q = s.pl_att[abase + e - nba];
-        j = __float_as_int(q.x);
-        r0 = q.y;
-        eps = q.z;
-        t = 2;
-      }
-      const float4 xj = X(j);
-      float lx, ly, lz;
-      float dx = diff_exact(xj.x, xi.x, lx), dy = diff_exact(xj.y, xi.y, ly),
-            dz = diff_exact(xj.z, xi.z, lz);
-      if (wrap) min_image3(dx, dy, dz, boxl);
-      const float cc = small_coeff(s, t, dx, dy, dz, lx, ly, lz, r0, eps, fene_bad);
-      acc3(ax[c], ay[c], az[c], cc, dx, dy, dz);
-    }
-  }
-
-  // Non-native repulsion, kC loads in flight per lane per chunk of kV entries
-  const RepConst rc = rep_const(s);
-  // pair-list partners are stored relative to the molecule's first bead
-  const unsigned short* __restrict__ prow = s.pl_j + rbase;
-  const int jbase = s.mol[m1].start;
-  for (int base = 0; base < rcnt; base += kV) {
-    int jj[kC];
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      const int e = base + lane + c * G;
-      jj[c] = e < rcnt ? jbase + (int)prow[e] : i;
-    }
-    float4 xx[kC];
-#pragma unroll
-    for (int c = 0; c < kC; ++c) xx[c] = X(jj[c]);
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      // past the row end xx[c] is bead i itself: d2 = 0 fails the tolerance
-      // test and contributes exactly 0, so no branch is needed
-      rep_entry<UNI, wrap>(rc, xi, xx[c], ax[c], ay[c], az[c]);
-    }
-  }
-  // upper levels of the fixed tree inside the lane, lower levels by shuffles
-#pragma unroll
-  for (int off = kV / 2; off >= G; off >>= 1) {
-    const int oc = off / G;
-#pragma unroll
-    for (int c = 0; c < kC; ++c)
-      if (c < oc) {
-        ax[c] = __fadd_rn(ax[c], ax[c + oc]);
-        ay[c] = __fadd_rn(ay[c], ay[c + oc]);
-        az[c] = __fadd_rn(az[c], az[c + oc]);
-      }
-  }
-#pragma unroll
-  for (int off = G / 2; off > 0; off >>= 1) {
-    ax[0] = __fadd_rn(ax[0], __shfl_xor_sync(gmask, ax[0], off));
-    ay[0] = __fadd_rn(ay[0], __shfl_xor_sync(gmask, ay[0], off));
-    az[0] = __fadd_rn(az[0], __shfl_xor_sync(gmask, az[0], off));
-  }
-  fene_bad = __any_sync(gmask, fene_bad);
-  fx = ax[0];
-  fy = ay[0];
-  fz = az[0];
-}
-
-// wrap is 0 when no pair of the molecule can reach boxl/4 (from its last
-// binning, with a cut-off of margin): the minimum image is then the identity.
-// The test of every entry then costs more than its arithmetic saves branches,
-// so the sum is compiled for both.
-template <int G, bool UNI, class XS>
-__device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, int lane,
-                                           int2 br, int2 ar, int abase, int acnt, int rcnt,
-                                           float& fx, float& fy, float& fz, bool& fene_bad) {
-  if (s.grid[m1].wrap)
-    bead_force_w<G, UNI, true>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
-  else
-    bead_force_w<G, UNI, false>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
-}
-
 // SPLIT = false: one kernel -- the groups' sums go through shared memory to
 // one thread per bead, which completes the step (finish_bead).  SPLIT = true:
 // the sums go to s.fsum and k_finish completes the step in a second launch

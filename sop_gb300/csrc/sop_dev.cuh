@@ -80,6 +80,8 @@ struct DevSys {
   unsigned seed_lo, seed_hi;
 
   float4* x[2];
+  float4* xl[2];                // the last completed step's coordinates at its parity (contexts
+                                // that rebuild the pair list and step in one launch)
   float4* p[2];
   float4* v;
   float4* incr;
@@ -117,6 +119,28 @@ struct DevSys {
   float4* noise;                // injected normals or nullptr
   int use_noise;
 };
+
+// Tables of the tile step (kernels_tile.cu), rebuilt after every pair-list
+// rebuild; a tile is `beads` consecutive bead slots.
+constexpr int kTileCap = 2048;     // distinct beads a tile may touch
+constexpr int kTileChunks = 12;    // chunks of 16 entries of a repulsive row
+constexpr int kTileSmall = 32;     // bonded, angle and native entries of a bead
+constexpr int kTileWords = 512;    // 32-bead words from a tile's first to its last molecule's end
+                                   // (a tile's context has at most 16,384 beads)
+constexpr int kTileSmemMost = 50 * 1024;
+struct TileSet {
+  int beads, ntile;
+  int smem;             // dynamic shared memory of a block
+  int* cnt;             // distinct beads of each tile; -1: its lists do not fit
+  int* bead;            // those beads, ascending: kTileCap per tile
+  int2* dim;            // {longest row in chunks | most small entries << 16, list position of its first bead}
+  int* num;             // per bead: small entries | row chunks << 16
+  unsigned short* rep;  // repulsive rows as list positions: kTileChunks * 16 * beads per tile
+  float4* small;        // {r0, eps, list position, type} [entry][bead]: kTileSmall * beads per tile
+};
+__host__ __device__ constexpr int tile_smem(int beads, int cnt, int chunks, int small) {
+  return 16 * cnt + 16 * beads * small + 32 * beads * chunks;
+}
 
 enum { FLAG_NL_OVERFLOW = 1, FLAG_BARRIER_TIMEOUT = 2 };
 
