@@ -796,6 +796,9 @@ void set_constants(SopCtx* ctx) {
       if (a > 0 && b > 0) rcmax = std::max(rcmax, rcut_of(P.nl_rep_fac, P.nl_rep_abs, sg));
     }
   s.rc_nl_rep_max = rcmax;
+  // lists rebuilt rarely or never let pairs drift further before the next look
+  // at the extent: there the flag keeps twice the margin
+  s.wrap_from = P.nnlup > 0 && P.nnlup <= 200 ? 0.5f : 0.25f;
   s.seed_lo = (unsigned)(P.seed & 0xffffffffULL);
   s.seed_hi = (unsigned)(P.seed >> 32);
 }

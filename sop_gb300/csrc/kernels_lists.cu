@@ -169,11 +169,11 @@ __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsig
   bool periodic = false;
   for (int a = 0; a < 3; ++a) periodic |= !(ext[a] + rc < s.boxl);  // also true for NaN extents
   // Separations inside the box [lo, lo + ext] never exceed ext (rounding is
-  // monotone), so below boxl/4 the minimum image leaves them unchanged.  The
-  // margin of one cut-off covers the drift until the next rebuild, for the
-  // pair-list filters that use the same flag.
+  // monotone), and below boxl/2 the minimum image leaves them unchanged
+  // (rint(d / boxl) is 0).  The margin of one cut-off covers the drift until the
+  // next rebuild, for the steps and pair-list filters that use the same flag.
   bool wrap = false;
-  for (int a = 0; a < 3; ++a) wrap |= !(ext[a] + rc < 0.25f * s.boxl);
+  for (int a = 0; a < 3; ++a) wrap |= !(ext[a] + rc < s.wrap_from * s.boxl);
   if (periodic || n <= 96) {
     g.brute = 1;
   } else {
@@ -213,6 +213,11 @@ __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsig
     g.lo[0] = g.lo[1] = g.lo[2] = 0.0f;
   }
   g.wrap = wrap ? 1 : 0;
+  // A molecule that cannot come within a cut-off of its own image is binned by
+  // plain separations, and lists pairs within a cut-off of each other only:
+  // their separations stay below boxl/2 however far the molecule reaches (a
+  // 50,000-bead globule, 340 A across, in a box of 500 A).
+  g.wrap_list = wrap && (g.brute || s.wrap_from < 0.5f || !(4.1f * rc < s.boxl)) ? 1 : 0;
   g.ncell = g.dims[0] * g.dims[1] * g.dims[2];
   g.base = base;
   return g;
@@ -493,7 +498,7 @@ __global__ void __launch_bounds__(kNlThreads, 4) k_nl(DevSys s, int koff) {
   const int y0 = max(cy - g.S, 0), y1 = min(cy + g.S, ny - 1);
   const int x0 = max(cx - g.S, 0), x1 = min(cx + g.S, nx - 1);
   const float boxl = s.boxl;
-  const bool wrap = g.wrap != 0;
+  const bool wrap = g.wrap_list != 0;
   const float inv_cs = g.brute ? 0.0f : 1.0f / g.cs;
   const float r11 = s.rc2_nl_rep[1][1], r12 = s.rc2_nl_rep[1][2], r22 = s.rc2_nl_rep[2][2];
   const float rcm = s.rc_nl_rep_max * 1.0001f + 1.0e-3f;
@@ -637,8 +642,8 @@ __global__ void __launch_bounds__(256, 5) k_pl(DevSys s, int koff) {  // 48 regi
   const int m = s.mol_of[i];
   if (!mol_listed(s, m, koff)) return;  // finished or stopped: keeps the lists of its last step
   int nrep, natt;
-  pair_rows<UNI, L>(
-      s, xbuf(s, m, koff), i, pair_head<L>(s, i, m), [](int, int) {}, [](int, float4) {}, nrep, natt);
+  pair_rows<UNI, L, false>(
+      s, xbuf(s, m, koff), i, pair_head<L, false>(s, i, m), [](int, int) {}, [](int, float4) {}, nrep, natt);
 }
 
 // ------------------------------------------------------------ host side

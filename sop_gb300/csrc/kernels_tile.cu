@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_pl_tile(DevSys s, TileSet ts,
     const int2 br = s.bond_row[i], ar = s.ang_row[i];
     int nrep, natt;
     if (!only_tables && mol_listed(s, m, koff)) {
-      pair_rows<UNI, 32>(
-          s, xbuf(s, m, koff), i, pair_head<32>(s, i, m), [&](int, int j) { mark(start + j); },
+      pair_rows<UNI, 32, false>(
+          s, xbuf(s, m, koff), i, pair_head<32, false>(s, i, m), [&](int, int j) { mark(start + j); },
           [&](int, float4 a) { mark(__float_as_int(a.x)); }, nrep, natt);
     } else {  // the rows stay as they are
       nrep = s.pl_cnt[i];
@@ -178,9 +178,9 @@ __global__ void __launch_bounds__(kBuildThreads) k_pl_tile(DevSys s, TileSet ts,
 // -------------------------------------------------------------------- step
 // The force on a tile's bead from the staged tables, G lanes a bead: lane
 // `lane` of G sums virtual lanes lane + c * G (the order of bead_force).
-template <int TB, bool UNI, bool wrap>
+template <int TB, bool UNI, bool wrap_list>
 __device__ __forceinline__ void tile_force(const DevSys& s, const float4* x, const float4* small,
-                                           const unsigned short* rep, int q, int self, int nsmall,
+                                           const unsigned short* rep, bool wrap, int q, int self, int nsmall,
                                            int chunks, int lane, float& fx, float& fy, float& fz,
                                            bool& fene_bad) {
   constexpr int G = kTileThreads / TB, kC = kV / G;
@@ -222,7 +222,7 @@ __device__ __forceinline__ void tile_force(const DevSys& s, const float4* x, con
 #pragma unroll
     for (int c = 0; c < kC; ++c) xx[c] = x[j[c]];
 #pragma unroll
-    for (int c = 0; c < kC; ++c) rep_entry<UNI, wrap>(rc, xi, xx[c], ax[c], ay[c], az[c]);
+    for (int c = 0; c < kC; ++c) rep_entry<UNI, wrap_list>(rc, xi, xx[c], ax[c], ay[c], az[c]);
   }
   group_sum<G>(ax, ay, az, fx, fy, fz, fene_bad);
 }
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
   uint4* const rtable = reinterpret_cast<uint4*>(stable + small * TB);
   int num = 0, m = 0;
   long long n = 0;
-  bool run = false, wrap = false;
+  bool run = false, wrap = false, wrap_list = false;
   if (q < nb) {
     m = s.mol_of[b0 + q];
     num = ts.num[b0 + q];
@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
     n = s.mol_step[m] + 1 + koff;
     run = mc.active && n >= 0 && !(mc.nsteps >= 0 && n > mc.nsteps) && !frozen;
     wrap = s.grid[m].wrap != 0;
+    wrap_list = s.grid[m].wrap_list != 0;
   }
   // a listed bead's coordinates at its own molecule's step
   auto source = [&](int b) {
@@ -318,11 +319,11 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
   if (run) {
     if (cnt >= 0) {
       const unsigned short* rep = reinterpret_cast<const unsigned short*>(rtable);
-      if (wrap)
-        tile_force<TB, UNI, true>(s, dyn, stable, rep, q, dim.y + q, num & 0xffff, num >> 16, lane,
+      if (wrap_list)
+        tile_force<TB, UNI, true>(s, dyn, stable, rep, wrap, q, dim.y + q, num & 0xffff, num >> 16, lane,
                                   fx, fy, fz, bad);
       else
-        tile_force<TB, UNI, false>(s, dyn, stable, rep, q, dim.y + q, num & 0xffff, num >> 16, lane,
+        tile_force<TB, UNI, false>(s, dyn, stable, rep, wrap, q, dim.y + q, num & 0xffff, num >> 16, lane,
                                    fx, fy, fz, bad);
     } else {
       const int i = b0 + q;
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
     other = (int)(n & 1) != par;
     br = s.bond_row[i];
     ar = s.ang_row[i];
-    head = pair_head<G>(s, i, m);
+    head = pair_head<G, true>(s, i, m);
     if (lane < br.y) {
       j0 = s.bond_j[br.x + lane];
       r0 = s.bond_r0[br.x + lane];
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
   // the bead's rows by the last step's coordinates XL, its force at the step's X
   auto bead = [&](const float4* XL, const float4* X) {
     int nrep, natt;
-    pair_rows<UNI, G>(
+    pair_rows<UNI, G, true>(
         s, XL, i, head,
         [&](int pos, int j) {
           if (pos < kPairRep) rrow[q][pos] = (unsigned short)j;
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
     float ax[kC] = {}, ay[kC] = {}, az[kC] = {};
     const int nba = br.y + ar.y, nsmall = nba + natt;
     auto sum = [&](auto wrapped) {
-      constexpr bool wrap = decltype(wrapped)::value;
+      constexpr bool wrap_list = decltype(wrapped)::value;
       for (int base = 0; base < nsmall; base += kV) {
 #pragma unroll
         for (int c = 0; c < kC; ++c) {
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
           float lx, ly, lz;
           float dx = diff_exact(xj.x, xi.x, lx), dy = diff_exact(xj.y, xi.y, ly),
                 dz = diff_exact(xj.z, xi.z, lz);
-          if (wrap) min_image3(dx, dy, dz, s.boxl);
+          if (head.wrap) min_image3(dx, dy, dz, s.boxl);
           const float cc = small_coeff(s, type, dx, dy, dz, lx, ly, lz, r, eps, bad);
           acc3(ax[c], ay[c], az[c], cc, dx, dy, dz);
         }
@@ -473,10 +474,10 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
         }
 #pragma unroll
         for (int c = 0; c < kB; ++c)  // past the row's end: the bead itself contributes 0
-          rep_entry<UNI, wrap>(rc, xi, xx[c], ax[c % kC], ay[c % kC], az[c % kC]);
+          rep_entry<UNI, wrap_list>(rc, xi, xx[c], ax[c % kC], ay[c % kC], az[c % kC]);
       }
     };
-    if (head.wrap) sum(std::true_type{});
+    if (head.wrap_list) sum(std::true_type{});
     else sum(std::false_type{});
     group_sum<G>(ax, ay, az, fx, fy, fz, bad);
   };

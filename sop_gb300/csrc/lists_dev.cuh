@@ -39,18 +39,19 @@ __device__ __forceinline__ unsigned group_mask(int wl) {
 // every entry of the two rows; nrep / natt are their lengths, in every lane.
 //
 // What the rebuild reads before any coordinate: the row lengths and the
-// first round of each row.  Only neighbour-list rebuilds write it, so a kernel
-// that follows others which use the lists may read it ahead of its wait.
+// first round of each row (of the attractive one when kAhead).  Only
+// neighbour-list rebuilds write it, so a kernel that follows others which use
+// the lists may read it ahead of its wait.
 struct PairHead {
   int cnt, acnt, mstart;
   int2 row;     // the bead's native row
-  bool wrap;    // from the neighbour-list build, with a cut-off of margin
+  bool wrap, wrap_list;  // from the neighbour-list build, with a cut-off of margin
   uint2 j;      // four entries of the repulsive row
   int natj;     // one of the attractive row: partner, squared cut-off, parameters
   float rc2;
   float4 par;
 };
-template <int L>
+template <int L, bool kAhead>
 __device__ __forceinline__ PairHead pair_head(const DevSys& s, int i, int m) {
   const int lane = threadIdx.x & (L - 1);
   PairHead h;
@@ -59,12 +60,13 @@ __device__ __forceinline__ PairHead pair_head(const DevSys& s, int i, int m) {
   h.row = s.nat_row[i];
   h.mstart = s.mol[m].start;
   h.wrap = s.grid[m].wrap != 0;
+  h.wrap_list = s.grid[m].wrap_list != 0;
   h.j = make_uint2(0, 0);
   if (4 * lane < h.cnt) h.j = reinterpret_cast<const uint2*>(s.nl_j + (long long)i * s.nl_stride)[lane];
   h.natj = 0;
   h.rc2 = 0.f;
   h.par = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (lane < h.acnt) {
+  if (kAhead && lane < h.acnt) {
     const int idx = s.nl_att_e[h.row.x + lane];
     h.natj = s.nat_j[idx];
     h.rc2 = s.nat_rc2[idx].y;
@@ -72,8 +74,8 @@ __device__ __forceinline__ PairHead pair_head(const DevSys& s, int i, int m) {
   }
   return h;
 }
-template <bool UNI, int L, class Rep, class Att>
-__device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int i, const PairHead& h,
+template <bool UNI, int L, bool kAhead, bool wrap_list, class Rep, class Att>
+__device__ __forceinline__ void pair_rows_w(const DevSys& s, const float4* X, int i, const PairHead& h,
                                           Rep rep, Att att, int& nrep, int& natt) {
   const int wl = threadIdx.x & 31;
   const int lane = wl & (L - 1);
@@ -81,7 +83,6 @@ __device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int 
   const float4 xi = X[i];
   const int ti = type_of(xi);
   const float boxl = s.boxl;
-  const bool wrap = h.wrap;
   const float r11 = s.rc2_pl_rep[1][1], r12 = s.rc2_pl_rep[1][2], r22 = s.rc2_pl_rep[2][2];
   const unsigned below = (1u << wl) - 1u;  // lanes of the warp before this one
   const long long a = (long long)i * s.nl_stride;
@@ -112,7 +113,7 @@ __device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int 
       const float4 xj = X[jq[q]];
       float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y),
             dz = __fsub_rn(xj.z, xi.z);
-      if (wrap) min_image3(dx, dy, dz, boxl);
+      if (wrap_list) min_image3(dx, dy, dz, boxl);
       const bool p = (e + q < cnt) &&
                      d2_exact(dx, dy, dz) < (UNI ? r11 : pick_type_pair(r11, r12, r22, ti, type_of(xj)));
       pb |= (p ? 1u : 0u) << q;
@@ -144,7 +145,7 @@ __device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int 
       j = h.natj;
       float rc2 = h.rc2;
       q = h.par;
-      if (e0 > 0) {
+      if (!kAhead || e0 > 0) {
         const int idx = s.nl_att_e[row.x + e];
         // the contact's partner, cut-off and parameters in one round of loads
         j = s.nat_j[idx];
@@ -154,7 +155,7 @@ __device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int 
       const float4 xj = X[j];
       float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y),
             dz = __fsub_rn(xj.z, xi.z);
-      if (wrap) min_image3(dx, dy, dz, boxl);
+      if (h.wrap) min_image3(dx, dy, dz, boxl);
       pass = d2_exact(dx, dy, dz) < rc2;
     }
     const unsigned mask = __ballot_sync(gmask, pass) & gmask;
@@ -169,6 +170,15 @@ __device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int 
   if (lane == 0) s.pl_att_cnt[i] = ka;
   nrep = k;
   natt = ka;
+}
+
+// Compiled with and without the minimum image of the repulsive pairs (the same
+// for a whole molecule).
+template <bool UNI, int L, bool kAhead, class Rep, class Att>
+__device__ __forceinline__ void pair_rows(const DevSys& s, const float4* X, int i, const PairHead& h,
+                                          Rep rep, Att att, int& nrep, int& natt) {
+  if (h.wrap_list) pair_rows_w<UNI, L, kAhead, true>(s, X, i, h, rep, att, nrep, natt);
+  else pair_rows_w<UNI, L, kAhead, false>(s, X, i, h, rep, att, nrep, natt);
 }
 
 }  // namespace sop

@@ -56,7 +56,8 @@ struct MolGrid {
   int base;                     // first cell
   int ncell;
   int brute;                    // 1: index-chunked cells, all pairs scanned
-  int wrap;                     // 0: no pair of the molecule can reach boxl/4 (no minimum image)
+  int wrap;                     // 0: no pair of the molecule can reach boxl/2 (no minimum image)
+  int wrap_list;                // 0: no pair of its repulsive lists can
 };
 
 struct DevSys {
@@ -72,6 +73,7 @@ struct DevSys {
   float rc2_nl_rep[3][3];       // squared cut-offs by type pair
   float rc2_pl_rep[3][3];
   float rc_nl_rep_max;          // max neighbour-list cut-off (A)
+  float wrap_from;              // fraction of boxl a separation stays below where the minimum image is left out
   float sig2[3][3];             // sigma_rep^2 by type pair
   float rep_tol[3][3];          // sigma_rep * 1e-7: pairs with d^2 <= this are skipped (energy.cu:555-558)
   int uniform_type;             // 1: every bead has type 1 (one sigma for all pairs)

@@ -76,8 +76,8 @@ __device__ __forceinline__ float small_coeff(const DevSys& s, int type, float dx
 // One non-native repulsion (energy.cu:536-581): co1 = -6 eps / d^2 (2 (s/r)^12 +
 // (s/r)^6) [rep6: -6 eps / d^2 (s/r)^6]; pairs with d^2 <= 1e-7 sigma are
 // skipped.  A system of one bead type (UNI) uses its sigma as a constant.
-// wrap is false when no pair of the molecule can reach boxl/4 (from its last
-// binning, with a cut-off of margin): the minimum image is then the identity.
+// wrap is false when no listed pair of the molecule can reach boxl/2 (from its
+// last binning, with a cut-off of margin): the minimum image is the identity.
 // (As a run-time test of every entry it cost 18% of the step's instructions
 // at 4 lanes per bead.)
 struct RepConst {

@@ -58,7 +58,7 @@ __device__ __forceinline__ void group_sum(float (&ax)[kV / G], float (&ay)[kV / 
 // ...).  Each physical lane holds kC = kV / G virtual lanes and does the
 // upper tree levels locally, the rest by shuffles.  So every G gives
 // bit-identical forces, and G is free to tune per context.
-template <int G, bool UNI, bool wrap, class XS>
+template <int G, bool UNI, bool wrap_list, class XS>
 __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i, int m1, int lane,
                                            int2 br, int2 ar, int abase, int acnt, int rcnt,
                                            float& fx, float& fy, float& fz, bool& fene_bad) {
@@ -68,6 +68,7 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
   for (int c = 0; c < kC; ++c) ax[c] = ay[c] = az[c] = 0.f;
   const float4 xi = X(i);
   const float boxl = s.boxl;
+  const bool wrap = s.grid[m1].wrap != 0;
   const long long rbase = (long long)i * s.nl_stride;
 
   // Bonded, angle and native terms share one index space [bonds | angles |
@@ -124,21 +125,19 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
     for (int c = 0; c < kC; ++c) {
       // past the row end xx[c] is bead i itself: d2 = 0 fails the tolerance
       // test and contributes exactly 0, so no branch is needed
-      rep_entry<UNI, wrap>(rc, xi, xx[c], ax[c], ay[c], az[c]);
+      rep_entry<UNI, wrap_list>(rc, xi, xx[c], ax[c], ay[c], az[c]);
     }
   }
   group_sum<G>(ax, ay, az, fx, fy, fz, fene_bad);
 }
 
-// wrap is 0 when no pair of the molecule can reach boxl/4 (from its last
-// binning, with a cut-off of margin): the minimum image is then the identity.
-// The test of every entry then costs more than its arithmetic saves branches,
-// so the sum is compiled for both.
+// Compiled with and without the minimum image of the repulsive pairs (the same
+// for a whole molecule).
 template <int G, bool UNI, class XS>
 __device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, int lane,
                                            int2 br, int2 ar, int abase, int acnt, int rcnt,
                                            float& fx, float& fy, float& fz, bool& fene_bad) {
-  if (s.grid[m1].wrap)
+  if (s.grid[m1].wrap_list)
     bead_force_w<G, UNI, true>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
   else
     bead_force_w<G, UNI, false>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);

@@ -134,3 +134,26 @@ def test_staged_after_upload_restore_and_noise(nplup):
             got += state(e)
         outs.append(got)
     same(*outs)
+
+
+@pytest.mark.parametrize("n,boxl", [(300, 90.0), (300, 130.0), (1500, 160.0), (4000, 190.0), (4000, 260.0),
+                                    (4000, 360.0)])
+@pytest.mark.parametrize("kw", [{}, dict(lanes_per_bead=4, step_split=2), dict(nplup=1)])
+def test_left_out_minimum_image(n, boxl, kw):
+    """Where the molecule's extent shows that the minimum image is the identity,
+    for every pair or for the listed ones, it is left out.  Contexts that rebuild
+    their lists rarely (nnlup > 200) keep it to a quarter of the box: over the
+    steps before either rebuilds them the results are the same bits, and the
+    lists equal the oracle's.  Boxes below, about and above twice the extent,
+    and ones the molecule reaches across."""
+    m = mol_of(n, 500 + n)
+    outs = []
+    for nnlup in (50, 1000):
+        p = engine.baseline_params(**{**dict(boxl=boxl, nnlup=nnlup), **kw})
+        with engine.plain(m, m.xyz, p, T=0.6) as e:
+            _, (nri, nrj), _, (opi, opj) = oracle_lists(m, m.xyz, p, boxl)
+            assert pairset(*e.list_pairs(0, 1)[:2]) == pairset(nri, nrj)
+            assert pairset(*e.list_pairs(0, 3)[:2]) == pairset(opi, opj)
+            e.step(45)
+            outs.append(state(e))
+    same(*outs)
