@@ -30,7 +30,7 @@ constexpr int kStepThreads = 128;  // small blocks: a finished block frees its S
 // Blocks per SM each lane-group width is compiled for (a register cap).
 template <int G>
 struct StepBlocks {
-  static constexpr int value = G == 4 ? 10 : (G == 8 ? 12 : (G == 16 ? 8 : 2));
+  static constexpr int value = G == 4 ? 10 : (G == 8 ? 10 : (G == 16 ? 8 : 2));
 };
 
 // STEP = false: force evaluation only at step mol_step + koff (velocities kept),
