@@ -19,7 +19,8 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["engine.cu", "kernels_lists.cu", "kernels_step.cu", "kernels_tile.cu", "energy_noalloc.cu"]
+CU_SOURCES = ["engine.cu", "kernels_lists.cu", "kernels_step.cu", "kernels_tile.cu", "kernels_io.cu",
+              "energy_noalloc.cu"]
 
 
 def nvcc() -> str:

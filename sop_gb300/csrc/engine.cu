@@ -22,6 +22,7 @@
 #include <thread>
 #include <vector>
 
+#include "io.cuh"
 #include "sop_dev.cuh"
 #include "../../include/sop_gpu.h"
 
@@ -58,8 +59,6 @@ cudaError_t launch_pair_step(const DevSys& s, int lanes, int koff, bool early, i
                              cudaStream_t st);
 void launch_gather_current(const DevSys& s, float* out, int* flag_out, cudaStream_t st);
 int energy_blocks(int mol_n);
-void launch_energy(const DevSys& s, int mol_start, int mol_n, int m, double* part, double* out,
-                   double k_bnd_R0sq_half, cudaStream_t st);
 void launch_observables(const DevSys& s, int mol_start, int mol_n, int m, int nnat,
                         double* part, double* out, cudaStream_t st);
 }  // namespace sop
@@ -218,8 +217,13 @@ struct SopCtx {
   long long bucket_beads[3] = {0, 0, 0};
   float ms_tiled = 0.f, ms_whole = 0.f;  // tuning times of the two step layouts
   double* e_part = nullptr;   // energy / observable partials
-  double* e_out = nullptr;    // 8 doubles
-  double* h_out = nullptr;    // pinned copy of e_out
+  int part_groups = 0;        // groups of partials in e_part
+  // pinned: [0..3] energy or observables, [8] flags, [9] a molecule's step, [10] its status
+  double* h_out = nullptr;
+  char* h_io = nullptr;       // pinned buffer of the transfers (kernels_io.cu), idle between calls
+  size_t io_bytes = 0;
+  float* d_io = nullptr;      // device buffer of the states of molecules above kPinnedBeads
+  bool queued = false;        // work was queued since the last wait that saw no overflow
   float4* stage = nullptr;    // gather buffer of sop_download_all
   // sop_download_all_async: two gather buffers (packed xyz, then the
   // overflow flag the gather saw), a copy stream, and per buffer the events
@@ -304,7 +308,9 @@ struct SopCtx {
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     if (h_out) cudaFreeHost(h_out);
+    if (h_io) cudaFreeHost(h_io);
     h_out = nullptr;
+    h_io = nullptr;
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
   }
@@ -487,22 +493,41 @@ int grow_nl(SopCtx* ctx) {
   return SOP_OK;
 }
 
-// Neighbour-list rebuild that regrows the rows on overflow and rebuilds
-// again; only_mol >= 0 rebuilds that molecule's lists alone.  Synchronous.
-int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol = -1) {
+// Waits for the stream and reads the flags.
+int wait_flags(SopCtx* ctx, int* flags) {
+  CK(cudaMemcpyAsync(ctx->h_out + 8, ctx->s.flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  std::memcpy(flags, ctx->h_out + 8, sizeof(int));
+  return SOP_OK;
+}
+
+// Neighbour-list rebuild, and what `then` queues behind it, that regrows the
+// rows on overflow and runs again; only_mol >= 0 rebuilds that molecule's
+// lists alone.  Synchronous.
+template <class F>
+int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol, F then) {
+  ctx->queued = true;
   for (int attempt = 0; attempt < 4; ++attempt) {
     DevSys s = ctx->s;  // re-read: a regrow changes the rows
     s.only_mol = only_mol;
     launch_nl_rebuild(s, ctx->w, koff, ctx->stream);
+    int rc = then(s);
+    if (rc) return rc;
     CK(cudaGetLastError());
     int flags = 0;
-    CK(cudaMemcpyAsync(&flags, ctx->s.flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (!(flags & FLAG_NL_OVERFLOW)) return SOP_OK;
-    int rc = grow_nl(ctx);
+    rc = wait_flags(ctx, &flags);
+    if (rc) return rc;
+    if (!(flags & FLAG_NL_OVERFLOW)) {
+      ctx->queued = false;
+      return SOP_OK;
+    }
+    rc = grow_nl(ctx);
     if (rc) return rc;
   }
   return ctx->fail(SOP_ERR_CAPACITY, "neighbour list kept overflowing");
+}
+int nl_rebuild_checked(SopCtx* ctx, int koff) {
+  return nl_rebuild_checked(ctx, koff, -1, [](const DevSys&) { return (int)SOP_OK; });
 }
 
 // Pair-list rebuild of the molecules of s, and of the tables the tile step
@@ -685,7 +710,7 @@ int graph_steps(const SopCtx* ctx) {
 // Queues nsteps steps of every molecule (no synchronisation).
 int step_async(SopCtx* ctx, long long nsteps) {
   const int P = graph_steps(ctx);
-  if (nsteps > 0) ctx->stepped = true;
+  if (nsteps > 0) ctx->stepped = ctx->queued = true;
   long long s0 = ctx->host_step;
   long long left = nsteps;
   while (left > 0) {
@@ -724,24 +749,28 @@ int barrier_failure(SopCtx* ctx) {
 }
 
 int sync_checked(SopCtx* ctx) {
-  for (int round = 0; round < 8; ++round) {
+  for (int round = 0; ctx->queued && round < 8; ++round) {
     int flags = 0;
-    CK(cudaMemcpyAsync(&flags, ctx->s.flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    int rc = wait_flags(ctx, &flags);
+    if (rc) return rc;
     if (flags & FLAG_BARRIER_TIMEOUT) return barrier_failure(ctx);
-    if (!(flags & FLAG_NL_OVERFLOW)) return SOP_OK;
+    if (!(flags & FLAG_NL_OVERFLOW)) {
+      ctx->queued = false;
+      return SOP_OK;
+    }
     // Every molecule froze at the neighbour-list rebuild that overflowed,
     // and the context's clock with them (enqueue_block advances the clocks
     // ahead of each such rebuild).
     long long done = 0;
     CK(cudaMemcpy(&done, ctx->s.sys_step, sizeof(long long), cudaMemcpyDeviceToHost));
-    int rc = grow_nl(ctx);
+    rc = grow_nl(ctx);
     if (rc) return rc;
     long long target = ctx->target_step;
     ctx->host_step = done;
     rc = step_async(ctx, target - done);
     if (rc) return rc;
   }
+  if (!ctx->queued) return SOP_OK;
   return ctx->fail(SOP_ERR_CAPACITY, "neighbour list kept overflowing");
 }
 
@@ -801,6 +830,20 @@ void set_constants(SopCtx* ctx) {
   s.wrap_from = P.nnlup > 0 && P.nnlup <= 200 ? 0.5f : 0.25f;
   s.seed_lo = (unsigned)(P.seed & 0xffffffffULL);
   s.seed_hi = (unsigned)(P.seed >> 32);
+}
+
+// States of molecules up to this many beads pass through pinned memory that the
+// kernels read and write in place, larger ones through device memory and one
+// copy per array: the host's own copy out of pinned memory takes 20 us for an
+// array of 50,000 beads, a copy from the device 4 us more than its wait.
+// us per download of 4 arrays, in place / copied: 500 beads 17 / 44, 8,000
+// 38 / 50, 16,000 64 / 53, 50,000 176 / 61.
+constexpr long long kPinnedBeads = 8192;
+constexpr size_t kServedIoBytes = 8u << 20;  // jobs that come and go together: about 30,000 beads
+
+int state_buffer(SopCtx* ctx, long long beads) {
+  if (!ctx->d_io) ctx->d_io = ctx->dalloc<float>(12 * (size_t)beads);
+  return ctx->d_io ? SOP_OK : ctx->fail(SOP_ERR_ALLOC, "state buffer allocation failed");
 }
 
 // Device arrays sized by capacities: beads, molecule slots, topology entries
@@ -865,17 +908,27 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   ctx->w.min_mol = (int)c.min_mol_beads;
   ctx->w.max_mol = (int)c.max_mol_beads;
   ctx->w.block_sums = ctx->dalloc<int>(scan_block_sums_needed(std::max<long long>(c.cells, nb)));
-  ctx->e_part = ctx->dalloc<double>(6 * (size_t)energy_blocks((int)c.max_mol_beads));
-  ctx->e_out = ctx->dalloc<double>(8);
+  // a served context sums the energies of all jobs that finish together
+  ctx->part_groups = energy_blocks((int)c.max_mol_beads) + (ctx->served ? 4096 : 0);
+  ctx->e_part = ctx->dalloc<double>(6 * (size_t)ctx->part_groups);
   if (!s.x[0] || !s.x[1] || !s.p[0] || !s.p[1] || !s.v || !s.incr || !s.f || !s.fsum || !s.mol_of ||
       !s.mol || !s.mol_step || !s.mol_status || !s.sys_step || !s.bond_row || !s.ang_row ||
       !s.nat_row || !s.bond_j || !s.bond_r0 || !s.ang_j || !s.nat_j || !s.nat_par ||
       !s.nat_rc2 || !s.nl_att_cnt || !s.pl_att_cnt || !s.nl_att_e || !s.pl_att || !s.nl_cnt ||
       !s.pl_cnt || !s.nl_maxrow || !s.bbox || !s.grid || !s.cell_cnt || !s.cell_start ||
       !s.cell_scan || !s.bead_cell || !s.bead_slot || !s.sorted || !s.xs || !s.flags ||
-      !ctx->w.block_sums || !ctx->e_part || !ctx->e_out)
+      !ctx->w.block_sums || !ctx->e_part)
     return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
-  if (!ctx->h_out) CK(cudaMallocHost(&ctx->h_out, 8 * sizeof(double)));
+  if (!ctx->h_out) CK(cudaMallocHost(&ctx->h_out, 16 * sizeof(double)));
+  if (!ctx->h_io) {
+    ctx->io_bytes = ctx->served ? std::max<size_t>(kServedIoBytes, 12 * nm)
+                                : 48 * (size_t)std::min<long long>(c.max_mol_beads, kPinnedBeads);
+    CK(cudaMallocHost(&ctx->h_io, ctx->io_bytes));
+  }
+  if (!ctx->served && c.max_mol_beads > kPinnedBeads) {
+    int rc = state_buffer(ctx, c.max_mol_beads);
+    if (rc) return rc;
+  }
   cudaStream_t st = ctx->stream;
   CK(cudaMemsetAsync(s.mol_of, 0xff, sizeof(int) * nb, st));   // -1: free
   CK(cudaMemsetAsync(s.fsum, 0, sizeof(float4) * nb, st));      // no step in flight
@@ -915,14 +968,22 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
 // so clearing tens of MB first would only cost time.
 template <class T>
 struct RawArray {
-  std::unique_ptr<T[]> p;
+  std::unique_ptr<T[]> own;
+  T* p = nullptr;
   size_t n = 0;
-  void reset(size_t k) {
-    p.reset(k ? new T[k] : nullptr);  // default-initialised: not cleared
+  // k entries: at *at, which moves on (16-byte steps), or its own
+  void reset(size_t k, char** at) {
+    if (at) {
+      p = reinterpret_cast<T*>(*at);
+      *at += (sizeof(T) * k + 15) / 16 * 16;
+    } else {
+      own.reset(k ? new T[k] : nullptr);  // default-initialised: not cleared
+      p = own.get();
+    }
     n = k;
   }
-  T* data() { return p.get(); }
-  const T* data() const { return p.get(); }
+  T* data() { return p; }
+  const T* data() const { return p; }
   size_t size() const { return n; }
   bool empty() const { return n == 0; }
   T& operator[](size_t i) { return p[i]; }
@@ -1027,26 +1088,34 @@ void fill_rows(const SopCtx* ctx, const HostMol& hm, int k, long long step0, Sta
 }
 
 // Sizes S for `beads` beads, `b2` / `a2` / `n2` bond / angle / native entries
-// and `nm` molecules starting at the given pool positions and slot.
+// and `nm` molecules starting at the given pool positions and slot, in memory
+// of its own or from *at on (staged_bytes).
 void size_staged(Staged& S, long long o, long long ob, long long oa, long long on, int slot0,
-                 long long beads, long long b2, long long a2, long long n2, int nm) {
+                 long long beads, long long b2, long long a2, long long n2, int nm,
+                 char** at = nullptr) {
   S.o = o; S.ob = ob; S.oa = oa; S.on = on; S.slot0 = slot0;
-  S.brow.reset(beads); S.arow.reset(beads); S.nrow.reset(beads);
-  S.molof.reset(beads);
-  S.x0.reset(beads); S.p0.reset(beads); S.v0.reset(beads);
-  S.bj.reset(b2); S.br.reset(b2);
-  S.aj.reset(a2);
-  S.nj.reset(n2); S.np.reset(n2); S.nr.reset(n2);
+  S.brow.reset(beads, at); S.arow.reset(beads, at); S.nrow.reset(beads, at);
+  S.molof.reset(beads, at);
+  S.x0.reset(beads, at); S.p0.reset(beads, at); S.v0.reset(beads, at);
+  S.bj.reset(b2, at); S.br.reset(b2, at);
+  S.aj.reset(a2, at);
+  S.nj.reset(n2, at); S.np.reset(n2, at); S.nr.reset(n2, at);
   S.mc.assign(nm, MolConst{});
   S.step0.assign(nm, 0);
 }
 
+// At most the bytes that size_staged takes for molecule hm.
+size_t staged_bytes(const HostMol& hm) {
+  return 16 * 13 + 76 * (size_t)hm.n + 16 * hm.bi.size() + 8 * hm.ai.size() + 56 * hm.ni.size();
+}
+
 // One molecule: its ranges and rows, staged on the host.
-int stage_install(SopCtx* ctx, int slot, HostMol& hm, long long step0, Staged& S) {
+int stage_install(SopCtx* ctx, int slot, HostMol& hm, long long step0, Staged& S,
+                  char** at = nullptr) {
   int rc = take_ranges(ctx, slot, hm);
   if (rc) return rc;
   size_staged(S, hm.start, hm.off_b, hm.off_a, hm.off_n, slot, hm.n, 2LL * (long long)hm.bi.size(),
-              2LL * (long long)hm.ai.size(), 2LL * (long long)hm.ni.size(), 1);
+              2LL * (long long)hm.ai.size(), 2LL * (long long)hm.ni.size(), 1, at);
   fill_rows(ctx, hm, 0, step0, S);
   ctx->mc[slot] = S.mc[0];
   return SOP_OK;
@@ -1099,21 +1168,65 @@ int install(SopCtx* ctx, int slot, HostMol& hm, long long step0) {
   return upload_staged(ctx, S);
 }
 
-// Frees molecule slot `slot`: inactive on the device, its beads unowned,
-// its pool ranges returned.  The stream must be idle.
-int uninstall(SopCtx* ctx, int slot) {
+// Returns the pool ranges of molecule slot `slot`, which the device no longer
+// uses (k_retire).
+void release_slot(SopCtx* ctx, int slot) {
   HostMol& hm = ctx->mols[slot];
-  if (hm.start < 0) return SOP_OK;
-  MolConst off{};
-  CK(cudaMemcpy(ctx->dmol + slot, &off, sizeof(MolConst), cudaMemcpyHostToDevice));
-  CK(cudaMemset(ctx->s.mol_of + hm.start, 0xff, sizeof(int) * (size_t)hm.n));
   ctx->bead_alloc.release(hm.start, hm.n);
   ctx->bond_alloc.release(hm.off_b, 2LL * (long long)hm.bi.size());
   ctx->ang_alloc.release(hm.off_a, 2LL * (long long)hm.ai.size());
   ctx->nat_alloc.release(hm.off_n, 2LL * (long long)hm.ni.size());
   ctx->mc[slot] = MolConst{};
-  hm.start = -1;
+  hm = HostMol();
   ctx->free_slots.push_back(slot);
+}
+
+// Molecules on their way into their slots, their rows in the pinned buffer.
+struct Arrivals {
+  int count = 0, most = 0;  // molecules; beads of the largest
+  size_t used = 0;
+};
+constexpr int kArrivals = 256;  // most together
+
+// Queues the installation of the molecules collected so far.
+int flush_arrivals(SopCtx* ctx, Arrivals& a) {
+  if (!a.count) return SOP_OK;
+  ctx->queued = true;
+  launch_install(ctx->s, ctx->dmol, reinterpret_cast<const InstallJob*>(ctx->h_io), a.count, a.most,
+                 ctx->stream);
+  CK(cudaGetLastError());
+  a = Arrivals{};
+  return SOP_OK;
+}
+
+// One molecule into slot `slot` by the next flush, its step counter at step0.
+int collect_arrival(SopCtx* ctx, int slot, HostMol& hm, long long step0, Arrivals& a) {
+  const size_t table = kArrivals * sizeof(InstallJob), need = staged_bytes(hm);
+  if (table + need > ctx->io_bytes) return install(ctx, slot, hm, step0);
+  if (a.count == kArrivals || table + a.used + need > ctx->io_bytes) {
+    int rc = flush_arrivals(ctx, a);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(ctx->stream));  // the buffer is filled anew
+  }
+  Staged S;
+  char *const from = ctx->h_io + table + a.used, *at = from;
+  int rc = stage_install(ctx, slot, hm, step0, S, &at);
+  if (rc) return rc;
+  InstallJob& j = reinterpret_cast<InstallJob*>(ctx->h_io)[a.count];
+  j.n = hm.n;
+  j.nb = (int)S.bj.size(); j.na = (int)S.aj.size(); j.nn = (int)S.nj.size();
+  j.slot = slot;
+  j.o = S.o; j.ob = S.ob; j.oa = S.oa; j.on = S.on;
+  j.step0 = step0;
+  j.mc = S.mc[0];
+  auto words = [](const auto& v) { return reinterpret_cast<const float*>(v.data()); };
+  j.x0 = words(S.x0); j.p0 = words(S.p0); j.v0 = words(S.v0);
+  j.brow = S.brow.data(); j.arow = S.arow.data(); j.nrow = S.nrow.data();
+  j.bj = S.bj.data(); j.aj = S.aj.data(); j.nj = S.nj.data();
+  j.br = S.br.data(); j.np = words(S.np); j.nr = words(S.nr);
+  a.used += at - from;
+  ++a.count;
+  a.most = std::max(a.most, hm.n);
   return SOP_OK;
 }
 
@@ -1339,19 +1452,11 @@ int check_mol(SopCtx* ctx, int mol) {
   return SOP_OK;
 }
 
-int read_step(SopCtx* ctx, int mol, long long* step) {
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->s.mol_step + mol, sizeof(long long), cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  std::memcpy(step, ctx->h_out, sizeof(long long));
-  return SOP_OK;
-}
-
-// float4 device rows -> 3 floats per bead on the host
-int copy3(SopCtx* ctx, float* dst, const float4* src, int n) {
-  CK(cudaMemcpy2DAsync(dst, 3 * sizeof(float), src, sizeof(float4), 3 * sizeof(float), n,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-  return SOP_OK;
+// The energy terms of molecule slot m.
+void energy_async(SopCtx* ctx, int m) {
+  const HostMol& hm = ctx->mols[m];
+  launch_energy(ctx->s, EnergyJob{hm.start, hm.n, m, 0}, nullptr, 1, ctx->e_part, ctx->h_out,
+                0.5 * ctx->P.k_bnd * ctx->P.R0 * ctx->P.R0, ctx->stream);
 }
 
 }  // namespace
@@ -1475,34 +1580,61 @@ static int make_hostmol(SopCtx* ctx, const sop_molecule* m, HostMol& h) {
 }
 
 // ------------------------------------------------------------- serving
-static int retire(SopCtx* ctx, int slot, const std::vector<long long>& steps,
+// Takes the results of the jobs in `slots` to the host and frees the slots, as
+// many jobs at a time as the pinned buffer and the partial sums hold (any one
+// job fits): their table, their energies, their states.
+static int retire(SopCtx* ctx, const std::vector<int>& slots, const std::vector<long long>& steps,
                   const std::vector<int>& status) {
-  Job& jb = ctx->jobs[ctx->slot_job[slot]];
-  HostMol& hm = ctx->mols[slot];
-  const long long st = std::max<long long>(steps[slot], 0);
-  const int cur = (int)(st & 1);
-  jb.unc.resize(3 * (size_t)hm.n);
-  jb.vel.resize(3 * (size_t)hm.n);
-  int rc = copy3(ctx, jb.unc.data(), ctx->s.x[cur] + hm.start, hm.n);
-  if (rc) return rc;
-  rc = copy3(ctx, jb.vel.data(), ctx->s.v + hm.start, hm.n);
-  if (rc) return rc;
-  launch_energy(ctx->s, hm.start, hm.n, slot, ctx->e_part, ctx->e_out,
-                0.5 * ctx->P.k_bnd * ctx->P.R0 * ctx->P.R0, ctx->stream);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->e_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  for (int t = 0; t < 4; ++t) jb.energy[t] = ctx->h_out[t];
-  jb.energy[4] = jb.energy[0] + jb.energy[1] + jb.energy[2] + jb.energy[3];
-  jb.status = status[slot] | (st >= jb.nsteps ? SOP_MOL_DONE : 0);
-  jb.steps = st;
-  jb.t_done = now_seconds();
-  jb.state = Job::FINISHED;
-  ctx->finished_new.push_back(ctx->slot_job[slot]);
-  rc = uninstall(ctx, slot);
-  if (rc) return rc;
-  ctx->slot_job[slot] = -1;
-  hm = HostMol();
+  for (size_t k0 = 0; k0 < slots.size();) {
+    size_t k1 = k0, bytes = 0;
+    int groups = 0, most = 0;
+    for (; k1 < slots.size() && k1 - k0 < 4096; ++k1) {
+      const int n = ctx->mols[slots[k1]].n;
+      const size_t more = sizeof(RetireJob) + 4 * sizeof(double) + 24 * (size_t)n;
+      if (bytes + more > ctx->io_bytes || groups + energy_blocks(n) > ctx->part_groups) break;
+      bytes += more;
+      groups += energy_blocks(n);
+      most = std::max(most, n);
+    }
+    const int count = (int)(k1 - k0);
+    RetireJob* tab = reinterpret_cast<RetireJob*>(ctx->h_io);
+    double* energy = reinterpret_cast<double*>(tab + count);
+    float* at = reinterpret_cast<float*>(energy + 4 * count);
+    groups = 0;
+    for (int k = 0; k < count; ++k) {
+      const int slot = slots[k0 + k];
+      const HostMol& hm = ctx->mols[slot];
+      tab[k].e = EnergyJob{hm.start, hm.n, slot, groups};
+      tab[k].cur = (int)(std::max<long long>(steps[slot], 0) & 1);
+      tab[k].unc = at;
+      tab[k].vel = at + 3 * (size_t)hm.n;
+      at += 6 * (size_t)hm.n;
+      groups += energy_blocks(hm.n);
+    }
+    launch_energy(ctx->s, EnergyJob{0, most, 0, 0}, tab, count, ctx->e_part, energy,
+                  0.5 * ctx->P.k_bnd * ctx->P.R0 * ctx->P.R0, ctx->stream);
+    launch_retire(ctx->s, ctx->dmol, tab, count, most, ctx->stream);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    for (int k = 0; k < count; ++k) {
+      const int slot = slots[k0 + k];
+      Job& jb = ctx->jobs[ctx->slot_job[slot]];
+      const size_t n3 = 3 * (size_t)ctx->mols[slot].n;
+      jb.unc.assign(tab[k].unc, tab[k].unc + n3);
+      jb.vel.assign(tab[k].vel, tab[k].vel + n3);
+      for (int t = 0; t < 4; ++t) jb.energy[t] = energy[4 * k + t];
+      jb.energy[4] = jb.energy[0] + jb.energy[1] + jb.energy[2] + jb.energy[3];
+      const long long st = std::max<long long>(steps[slot], 0);
+      jb.status = status[slot] | (st >= jb.nsteps ? SOP_MOL_DONE : 0);
+      jb.steps = st;
+      jb.t_done = now_seconds();
+      jb.state = Job::FINISHED;
+      ctx->finished_new.push_back(ctx->slot_job[slot]);
+      release_slot(ctx, slot);
+      ctx->slot_job[slot] = -1;
+    }
+    k0 = k1;
+  }
   return SOP_OK;
 }
 
@@ -1755,32 +1887,41 @@ static int serve_round(SopCtx* ctx) {
   const int nm = (int)ctx->caps.mols;
   std::vector<long long> steps(nm);
   std::vector<int> status(nm);
-  CK(cudaMemcpy(steps.data(), ctx->s.mol_step, sizeof(long long) * nm, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(status.data(), ctx->s.mol_status, sizeof(int) * nm, cudaMemcpyDeviceToHost));
+  char* const h_status = ctx->h_io + sizeof(long long) * nm;
+  CK(cudaMemcpyAsync(ctx->h_io, ctx->s.mol_step, sizeof(long long) * nm, cudaMemcpyDeviceToHost,
+                     ctx->stream));
+  CK(cudaMemcpyAsync(h_status, ctx->s.mol_status, sizeof(int) * nm, cudaMemcpyDeviceToHost,
+                     ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  std::memcpy(steps.data(), ctx->h_io, sizeof(long long) * nm);
+  std::memcpy(status.data(), h_status, sizeof(int) * nm);
+  std::vector<int> leaving;
   for (int slot = 0; slot < nm; ++slot) {
     const int id = ctx->slot_job[slot];
-    if (id < 0) continue;
-    if (status[slot] != 0 || steps[slot] >= ctx->jobs[id].nsteps) {
-      rc = retire(ctx, slot, steps, status);
-      if (rc) return rc;
-    }
+    if (id >= 0 && (status[slot] != 0 || steps[slot] >= ctx->jobs[id].nsteps))
+      leaving.push_back(slot);
   }
+  rc = retire(ctx, leaving, steps, status);
+  if (rc) return rc;
   // admission in arrival order; a job that does not fit yet lets the next
   // few (smaller) ones try
   int looked = 0;
   bool rebin = false;
+  Arrivals arrivals;
   for (auto it = ctx->queue.begin(); it != ctx->queue.end() && looked < 64 && !ctx->free_slots.empty();) {
     Job& jb = ctx->jobs[*it];
     const int slot = ctx->free_slots.back();
-    ctx->mols[slot] = jb.mol;
-    for (int t : jb.mol.types)
+    ctx->mols[slot] = std::move(jb.mol);
+    for (int t : ctx->mols[slot].types)
       if (t != 1 && ctx->s.uniform_type) {
         ctx->s.uniform_type = 0;
         ctx->drop_graphs();  // kernel arguments changed
       }
     const bool resumed = !jb.resume.empty();
-    rc = install(ctx, slot, ctx->mols[slot], resumed ? jb.resume_step : -(long long)ctx->P.nnlup);
+    rc = resumed ? install(ctx, slot, ctx->mols[slot], jb.resume_step)
+                 : collect_arrival(ctx, slot, ctx->mols[slot], -(long long)ctx->P.nnlup, arrivals);
     if (rc == SOP_ERR_CAPACITY) {
+      jb.mol = std::move(ctx->mols[slot]);
       ctx->mols[slot] = HostMol();
       ++it;
       ++looked;
@@ -1800,9 +1941,10 @@ static int serve_round(SopCtx* ctx) {
     ctx->slot_job[slot] = *it;
     jb.slot = slot;
     jb.state = Job::ACTIVE;
-    jb.mol = HostMol();
     it = ctx->queue.erase(it);
   }
+  rc = flush_arrivals(ctx, arrivals);
+  if (rc) return rc;
   update_live(ctx);
   if (rebin) {
     launch_rebin(ctx->s, ctx->w, ctx->stream);
@@ -1986,46 +2128,33 @@ int sop_upload_state(void* p, int mol, const float* pos, const float* unc_pos, c
   if (rc) return rc;
   rc = sync_checked(ctx);
   if (rc) return rc;
-  long long step;
-  rc = read_step(ctx, mol, &step);
-  if (rc) return rc;
   const HostMol& hm = ctx->mols[mol];
-  const int cur = (int)(step & 1);
-  std::vector<float4> buf(hm.n);
-  std::vector<float4> old(hm.n);
-  CK(cudaMemcpy(old.data(), ctx->s.x[cur] + hm.start, sizeof(float4) * hm.n, cudaMemcpyDeviceToHost));
   // the new state goes to both coordinate buffers: the lists are rebuilt from
   // it at block offset -1 (before this step's force evaluation), and the
   // force evaluation reads buffer step & 1
-  if (unc_pos) {
-    for (int i = 0; i < hm.n; ++i)
-      buf[i] = make_float4(unc_pos[3 * i], unc_pos[3 * i + 1], unc_pos[3 * i + 2], old[i].w);
-    for (int b = 0; b < 2; ++b)
-      CK(cudaMemcpy(ctx->s.x[b] + hm.start, buf.data(), sizeof(float4) * hm.n, cudaMemcpyHostToDevice));
+  const bool pinned = hm.n <= kPinnedBeads;
+  if (!pinned && (rc = state_buffer(ctx, ctx->caps.max_mol_beads))) return rc;
+  float* at = pinned ? reinterpret_cast<float*>(ctx->h_io) : ctx->d_io;
+  const size_t n3 = 3 * (size_t)hm.n;
+  const float* src[3] = {pos, unc_pos, vel};
+  float* in[3] = {};
+  for (int a = 0; a < 3; ++a) {
+    if (!src[a]) continue;
+    in[a] = at;
+    at += n3;
+    if (pinned) std::memcpy(in[a], src[a], sizeof(float) * n3);
+    else CK(cudaMemcpyAsync(in[a], src[a], sizeof(float) * n3, cudaMemcpyHostToDevice, ctx->stream));
   }
-  const float* pp = pos ? pos : unc_pos;
-  if (pp) {
-    for (int i = 0; i < hm.n; ++i) buf[i] = make_float4(pp[3 * i], pp[3 * i + 1], pp[3 * i + 2], 0.f);
-    for (int b = 0; b < 2; ++b)
-      CK(cudaMemcpy(ctx->s.p[b] + hm.start, buf.data(), sizeof(float4) * hm.n, cudaMemcpyHostToDevice));
-  }
-  if (vel) {
-    for (int i = 0; i < hm.n; ++i) buf[i] = make_float4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], 0.f);
-    CK(cudaMemcpy(ctx->s.v + hm.start, buf.data(), sizeof(float4) * hm.n, cudaMemcpyHostToDevice));
-  }
+  launch_unpack_state(ctx->s, hm.start, hm.n, in[0] ? in[0] : in[1], in[1], in[2], ctx->stream);
   // the lists of this molecule alone: the others keep theirs (built from
   // their own step's coordinates; buffer step - 1 holds their look-ahead)
-  rc = nl_rebuild_checked(ctx, -1, mol);
-  if (rc) return rc;
-  DevSys one = ctx->s;
-  one.only_mol = mol;
-  rc = keep_last(ctx);
-  if (rc) return rc;
-  rebuild_pairs(ctx, one, -1);
-  force_eval_async(ctx);  // every molecule: the same forces again for the others
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(ctx->stream));
-  return SOP_OK;
+  return nl_rebuild_checked(ctx, -1, mol, [&](const DevSys& one) {
+    int e = keep_last(ctx);
+    if (e) return e;
+    rebuild_pairs(ctx, one, -1);
+    force_eval_async(ctx);  // every molecule: the same forces again for the others
+    return (int)SOP_OK;
+  });
 }
 
 int sop_step(void* p, long long nsteps) {
@@ -2048,6 +2177,7 @@ int sop_sync(void* p) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
+  ctx->queued = true;
   int rc = sync_checked(ctx);
   if (rc) return rc;
   if (ctx->copy_stream) CK(cudaStreamSynchronize(ctx->copy_stream));
@@ -2058,6 +2188,7 @@ int sop_launch_stage(void* p, int stage, int koff) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
+  ctx->queued = true;
   switch (stage) {
     case 0:
       if (ctx->pair_step) CK(launch_pair_step(ctx->s, ctx->pair_step, koff, false, ctx->w.max_mol, ctx->stream));
@@ -2157,16 +2288,26 @@ int sop_download(void* p, int mol, float* pos, float* unc_pos, float* vel, float
   if (rc) return rc;
   rc = sync_checked(ctx);
   if (rc) return rc;
-  long long step;
-  rc = read_step(ctx, mol, &step);
-  if (rc) return rc;
   const HostMol& hm = ctx->mols[mol];
-  const int cur = (int)(step & 1);
-  if (pos && (rc = copy3(ctx, pos, ctx->s.p[cur] + hm.start, hm.n))) return rc;
-  if (unc_pos && (rc = copy3(ctx, unc_pos, ctx->s.x[cur] + hm.start, hm.n))) return rc;
-  if (vel && (rc = copy3(ctx, vel, ctx->s.v + hm.start, hm.n))) return rc;
-  if (force && (rc = copy3(ctx, force, ctx->s.f + hm.start, hm.n))) return rc;
+  const bool pinned = hm.n <= kPinnedBeads;
+  if (!pinned && (rc = state_buffer(ctx, ctx->caps.max_mol_beads))) return rc;
+  float* at = pinned ? reinterpret_cast<float*>(ctx->h_io) : ctx->d_io;
+  const size_t n3 = 3 * (size_t)hm.n;
+  float* dst[4] = {pos, unc_pos, vel, force};
+  StateOut o{};
+  for (int a = 0; a < 4; ++a)
+    if (dst[a]) {
+      o.a[a] = at;
+      at += n3;
+    }
+  launch_pack_state(ctx->s, mol, hm.start, hm.n, o, ctx->stream);
+  CK(cudaGetLastError());
+  for (int a = 0; a < 4 && !pinned; ++a)
+    if (dst[a])
+      CK(cudaMemcpyAsync(dst[a], o.a[a], sizeof(float) * n3, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  for (int a = 0; a < 4 && pinned; ++a)
+    if (dst[a]) std::memcpy(dst[a], o.a[a], sizeof(float) * n3);
   return SOP_OK;
 }
 
@@ -2278,6 +2419,7 @@ int sop_download_all_async(void* p, float* unc_pos, long long* ticket) {
   if (!p || !unc_pos || !ticket) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
+  ctx->queued = true;
   if (!ctx->copy_stream) {
     CK(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
     for (int k = 0; k < 2; ++k) {
@@ -2332,11 +2474,8 @@ int sop_energy(void* p, int mol, double* terms) {
   if (rc) return rc;
   rc = sync_checked(ctx);
   if (rc) return rc;
-  const HostMol& hm = ctx->mols[mol];
-  launch_energy(ctx->s, hm.start, hm.n, mol, ctx->e_part, ctx->e_out,
-                0.5 * ctx->P.k_bnd * ctx->P.R0 * ctx->P.R0, ctx->stream);
+  energy_async(ctx, mol);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->e_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   for (int t = 0; t < 4; ++t) terms[t] = ctx->h_out[t];
   terms[4] = terms[0] + terms[1] + terms[2] + terms[3];  // rna_etot (energy.cu:76)
@@ -2351,10 +2490,9 @@ int sop_observables(void* p, int mol, double* out) {
   rc = sync_checked(ctx);
   if (rc) return rc;
   const HostMol& hm = ctx->mols[mol];
-  launch_observables(ctx->s, hm.start, hm.n, mol, (int)hm.ni.size(), ctx->e_part, ctx->e_out,
+  launch_observables(ctx->s, hm.start, hm.n, mol, (int)hm.ni.size(), ctx->e_part, ctx->h_out,
                      ctx->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->e_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   for (int t = 0; t < 4; ++t) out[t] = ctx->h_out[t];
   return SOP_OK;
@@ -2367,10 +2505,14 @@ int sop_molecule_status(void* p, int mol, int* status, long long* step) {
   if (rc) return rc;
   rc = sync_checked(ctx);
   if (rc) return rc;
-  long long st = 0;
-  int flags = 0;
-  CK(cudaMemcpy(&st, ctx->s.mol_step + mol, sizeof(long long), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(&flags, ctx->s.mol_status + mol, sizeof(int), cudaMemcpyDeviceToHost));
+  StateOut o{};
+  o.step = reinterpret_cast<long long*>(ctx->h_out + 9);
+  o.status = reinterpret_cast<int*>(ctx->h_out + 10);
+  launch_pack_state(ctx->s, mol, 0, 0, o, ctx->stream);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(ctx->stream));
+  const long long st = *o.step;
+  int flags = *o.status;
   const MolConst& mc = ctx->mc[mol];
   if (mc.nsteps >= 0 && st >= mc.nsteps) flags |= SOP_MOL_DONE;
   if (status) *status = flags;

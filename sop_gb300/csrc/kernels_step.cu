@@ -20,6 +20,7 @@
 // to track parity, and every molecule may sit at its own step.
 #include <algorithm>
 
+#include "io.cuh"
 #include "reduce_dev.cuh"
 #include "step_force.cuh"
 
@@ -421,9 +422,17 @@ __global__ void k_advance(DevSys s, int steps) {
 constexpr int kEnergyThreads = 128;
 constexpr int kTermBatch = 4;
 
-__global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, int mol_start, int mol_n, int m,
+//
+// A molecule, or with a table one per blockIdx.y (the jobs that a served context
+// finishes together: a launch of 12 us for all of them instead of one each).
+__global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, EnergyJob job,
+                                                            const RetireJob* __restrict__ jobs,
                                                             double* __restrict__ part) {
   __shared__ double red[4 * 32];
+  if (jobs) job = jobs[blockIdx.y].e;
+  const int mol_start = job.start, mol_n = job.n, m = job.m;
+  if ((int)blockIdx.x * kEnergyThreads >= mol_n) return;
+  part += 4 * (size_t)job.part;
   int i = mol_start + blockIdx.x * blockDim.x + threadIdx.x;
   float eb = 0.f, ea = 0.f, eat = 0.f, erp = 0.f;
   if (i < mol_start + mol_n) {
@@ -504,10 +513,16 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, int mol_sta
 constexpr int kFinalThreads = 256;
 
 __global__ void __launch_bounds__(kFinalThreads) k_energy_final(const double* __restrict__ part,
-                                                                 int nblocks, double k_bnd_R0sq_half,
+                                                                 EnergyJob job,
+                                                                 const RetireJob* __restrict__ jobs,
+                                                                 double k_bnd_R0sq_half,
                                                                  double* __restrict__ out) {
   __shared__ double red[4 * 32];
   pdl_wait();
+  if (jobs) job = jobs[blockIdx.y].e;
+  const int nblocks = (job.n + kEnergyThreads - 1) / kEnergyThreads;
+  part += 4 * (size_t)job.part;
+  out += 4 * blockIdx.y;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < nblocks; b += kFinalThreads)
 #pragma unroll
@@ -798,11 +813,12 @@ void launch_advance(const DevSys& s, int steps, cudaStream_t st) {
 // Blocks (and groups of partial sums) of an energy or observables launch.
 int energy_blocks(int mol_n) { return (int)cdiv(mol_n, kEnergyThreads); }
 
-void launch_energy(const DevSys& s, int mol_start, int mol_n, int m, double* part, double* out,
-                   double k_bnd_R0sq_half, cudaStream_t st) {
-  const int nb = energy_blocks(mol_n);
-  k_energy<<<nb, kEnergyThreads, 0, st>>>(s, mol_start, mol_n, m, part);
-  launch_pdl(k_energy_final, 1, kFinalThreads, st, (const double*)part, nb, k_bnd_R0sq_half, out);
+void launch_energy(const DevSys& s, const EnergyJob& e, const RetireJob* jobs, int count,
+                   double* part, double* out, double k_bnd_R0sq_half, cudaStream_t st) {
+  const dim3 blocks(std::max(1, energy_blocks(e.n)), count);
+  k_energy<<<blocks, kEnergyThreads, 0, st>>>(s, e, jobs, part);
+  launch_pdl(k_energy_final, dim3(1, count), kFinalThreads, st, (const double*)part, e, jobs,
+             k_bnd_R0sq_half, out);
 }
 
 void launch_observables(const DevSys& s, int mol_start, int mol_n, int m, int nnat, double* part,

@@ -161,10 +161,10 @@ __device__ __forceinline__ void pdl_release() {
 
 // Launch with programmatic stream serialisation (see pdl_wait).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block,
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned block,
                               cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
