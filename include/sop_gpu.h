@@ -75,7 +75,7 @@ typedef struct sop_params {
   int nplup;          /* pair-list cadence, steps */
   int rep6;           /* 0: eps (s^12/r^12 + s^6/r^6) as energy.cu:436-437; 1: eps (s/r)^6 */
   int device;         /* CUDA device ordinal (set device, param.cpp:387-390) */
-  int graph_steps;    /* steps per captured CUDA graph (0: the engine's default) */
+  int graph_steps;    /* steps per captured CUDA graph (0: 10, later whole list periods) */
   int lanes_per_bead; /* 0: autotuned; else 2, 4, 8 or 16 (others: SOP_ERR_ARG) */
   unsigned long long seed; /* Philox key (replaces setup_rng's seed, GPUvars.cu:417-453) */
   int integrator;     /* 0: underdamped Langevin (sop.cu:421-462); 1: overdamped,

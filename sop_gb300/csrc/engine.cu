@@ -250,6 +250,7 @@ struct SopCtx {
   long long host_step = 0;    // common step of plain / batched contexts
   long long target_step = 0;  // step every molecule should reach after the queued work
   std::map<std::string, Graph> graphs;
+  int short_graphs = 0;       // launched graphs of graph_steps steps, up to kShortGraphs
   std::vector<MolConst> mc;
 
   ~SopCtx() { release(); }
@@ -292,6 +293,7 @@ struct SopCtx {
       if (kv.second.g) cudaGraphDestroy(kv.second.g);
     }
     graphs.clear();
+    short_graphs = 0;
   }
   void release() {
     if (copy_stream) cudaStreamSynchronize(copy_stream);  // copies into caller memory
@@ -707,21 +709,38 @@ int graph_steps(const SopCtx* ctx) {
   return P;
 }
 
+// A context that goes on stepping takes graphs of a whole neighbour-list period:
+// between two graphs lie the clock advance and the start of the next, 6 us, but a
+// period of 50 steps takes 150 us longer to capture than blocks of 10, so it is
+// captured once 40 of those have run (and would have paid for it).  us per pass
+// with blocks of 10 / 50 steps: 128 beads, 100 steps 535 / 484; 1,531 beads, 50
+// steps 590 / 568; 4,000 beads, 100 steps 797 / 769; 50,000 beads 1,475 / 1,461.
+// Not where the caller set the length, nor in served contexts, whose graphs are
+// captured again as jobs come and go.
+constexpr int kShortGraphs = 40, kMostGraphSteps = 100;
+int long_graph_steps(const SopCtx* ctx) {
+  const int P = graph_steps(ctx), L = ctx->P.nnlup;
+  return ctx->P.graph_steps <= 0 && !ctx->served && L > P && L % P == 0 && L <= kMostGraphSteps ? L : 0;
+}
+
 // Queues nsteps steps of every molecule (no synchronisation).
 int step_async(SopCtx* ctx, long long nsteps) {
-  const int P = graph_steps(ctx);
+  const int P = graph_steps(ctx), L = long_graph_steps(ctx);
   if (nsteps > 0) ctx->stepped = ctx->queued = true;
   long long s0 = ctx->host_step;
   long long left = nsteps;
   while (left > 0) {
     long long phase = s0 % P;
     if (phase == 0 && left >= P) {
+      const bool whole = L && s0 % L == 0 && left >= L && ctx->short_graphs >= kShortGraphs;
+      const int len = whole ? L : P;
+      if (!whole && ctx->short_graphs < kShortGraphs) ++ctx->short_graphs;
       cudaGraphExec_t ge;
-      int rc = graph_for(ctx, s0, P, &ge);
+      int rc = graph_for(ctx, s0, len, &ge);
       if (rc) return rc;
       CK(cudaGraphLaunch(ge, ctx->stream));
-      s0 += P;
-      left -= P;
+      s0 += len;
+      left -= len;
     } else {
       int cnt = (int)std::min<long long>(left, P - phase);
       enqueue_block(ctx, s0, cnt);

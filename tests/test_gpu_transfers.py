@@ -77,3 +77,23 @@ def test_jobs_past_the_buffer():
         one, = serve([t])
         for k in ("unc_pos", "vel", "energy", "status", "steps"):
             assert np.array_equal(together[t][k], one[k])
+
+
+@pytest.mark.parametrize("extra", [{}, dict(nplup=1), dict(nnlup=30, lanes_per_bead=4)])
+def test_period_graphs(extra):
+    """A context that goes on stepping takes graphs of a whole list period: the
+    same bits as blocks of 10, from any phase."""
+    ms = [system.generate(n, 13 + n) for n in (90, 300)]
+    got = []
+    for gs in (0, 10):
+        p = engine.baseline_params(graph_steps=gs, **extra)
+        with engine.Engine(p) as e:
+            for k, m in enumerate(ms):
+                e.add(m, m.xyz, traj=k, nsteps=640 if k else -1)
+            e.commit()
+            for n in (405, 5, 100, 49, 161):
+                e.step(n)
+            got.append([e.download(0), e.download(1), e.status(0), e.status(1), e.list_sizes()])
+    for a, b in zip(got[0][:2], got[1][:2]):
+        assert all(np.array_equal(a[k], b[k]) for k in a)
+    assert got[0][2:] == got[1][2:]
