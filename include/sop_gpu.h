@@ -89,8 +89,9 @@ typedef struct sop_params {
                          for plain and batched contexts of up to 16,384 bead
                          slots (with 0 or 1, and 0, 8 or 16 lanes per bead, its
                          reads are then staged in shared memory), by timing
-                         for larger ones (served contexts: 2).  Every form
-                         gives the same bits. */
+                         for larger ones (served contexts: 2 above 65,536 bead
+                         slots in use, else 1).  Every form gives the same
+                         bits. */
   int step_window;    /* shared-memory window of the step, in beads: each step
                          block stages the coordinates of its beads' molecules
                          (up to this many beads) and gathers partners from

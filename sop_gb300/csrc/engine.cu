@@ -1886,6 +1886,19 @@ bool ckpt_head(const void* buf, long long len, CkptHeader* h) {
          len == ckpt_bytes(h->n, h->cnt);
 }
 
+// The step of a served context by the bead slots its kernels cover: more lanes
+// and one kernel where they are few (lanes and form that the parameters set
+// stay).  us for a round of jobs with 4 lanes in two kernels / 8 lanes / 16 lanes:
+// 1,402 beads (slots: 12,800) 3,361 / 2,930 / 2,777; 8,470 (12,800) 5,467 / 4,739
+// / 4,543; 42,155 (51,000) 10,394 / 9,909 / 11,210; 98,390 (102,000) 19,353 /
+// 19,945 / 23,600.
+static void served_form(SopCtx* ctx) {
+  const int fixed_g = lanes_for(ctx), fixed_f = split_for(ctx);
+  const int n = ctx->s.nlive;
+  ctx->G = fixed_g ? fixed_g : n <= 16384 ? 16 : n <= 65536 ? 8 : 4;
+  ctx->split = fixed_f ? fixed_f != 1 : n > 65536;
+}
+
 // The per-step kernels of a served context cover the bead slots up to the
 // highest one in use, rounded up to a sixteenth of the pool: the step graphs
 // hold that bound, so they are re-captured only when it crosses a sixteenth.
@@ -1896,6 +1909,7 @@ static void update_live(SopCtx* ctx) {
   const long long live = std::min(cap, std::max(g, (hw + g - 1) / g * g));
   if (live != ctx->s.nlive) {
     ctx->s.nlive = (int)live;
+    served_form(ctx);
     ctx->drop_graphs();  // kernel arguments changed
   }
 }
@@ -2033,11 +2047,8 @@ int sop_serve_create(const sop_params* p, long long budget_bytes, long long max_
   ctx->mols.assign(c.mols, HostMol());
   ctx->slot_job.assign(c.mols, -1);
   // a served context fills up and empties as jobs come and go, so its step
-  // shape is fixed rather than timed once: 4 lanes per bead, two kernels
-  // (the faster form for a populated context) unless the parameters say
-  const int fixed_g = lanes_for(ctx), fixed_f = split_for(ctx);
-  ctx->G = fixed_g ? fixed_g : 4;
-  ctx->split = fixed_f != 1;
+  // shape follows a rule rather than being timed once
+  served_form(ctx);
   ctx->persist = false;
   ctx->one_block = false;
   CK(cudaStreamSynchronize(ctx->stream));
