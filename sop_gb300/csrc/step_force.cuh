@@ -79,29 +79,27 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
 #pragma unroll
     for (int c = 0; c < kC; ++c) {
       const int e = base + lane + c * G;
-      if (e >= nsmall) continue;
-      int j, t;
+      if (e >= nsmall) break;
+      int j;
       float r0 = 0.f, eps = 0.f;
       if (e < br.y) {
         j = s.bond_j[br.x + e];
         r0 = s.bond_r0[br.x + e];
-        t = 0;
       } else if (e < nba) {
         j = s.ang_j[ar.x + e - br.y];
-        t = 1;
       } else {
         const float4 q = s.pl_att[abase + e - nba];
         j = __float_as_int(q.x);
         r0 = q.y;
         eps = q.z;
-        t = 2;
       }
       const float4 xj = X(j);
       float lx, ly, lz;
       float dx = diff_exact(xj.x, xi.x, lx), dy = diff_exact(xj.y, xi.y, ly),
             dz = diff_exact(xj.z, xi.z, lz);
       if (wrap) min_image3(dx, dy, dz, boxl);
-      const float cc = small_coeff(s, t, dx, dy, dz, lx, ly, lz, r0, eps, fene_bad);
+      const float cc = small_coeff(s, e < br.y ? 0 : e < nba ? 1 : 2, dx, dy, dz, lx, ly, lz, r0,
+                                   eps, fene_bad);
       acc3(ax[c], ay[c], az[c], cc, dx, dy, dz);
     }
   }
