@@ -220,7 +220,7 @@ struct SopCtx {
   int part_groups = 0;        // groups of partials in e_part
   // pinned: [0..3] energy or observables, [8] flags, [9] a molecule's step, [10] its status
   double* h_out = nullptr;
-  char* h_io = nullptr;       // pinned buffer of the transfers (kernels_io.cu), idle between calls
+  char* h_io = nullptr;       // behind h_out: buffer of the transfers (kernels_io.cu), idle between calls
   size_t io_bytes = 0;
   float* d_io = nullptr;      // device buffer of the states of molecules above kPinnedBeads
   bool queued = false;        // work was queued since the last wait that saw no overflow
@@ -310,7 +310,6 @@ struct SopCtx {
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     if (h_out) cudaFreeHost(h_out);
-    if (h_io) cudaFreeHost(h_io);
     h_out = nullptr;
     h_io = nullptr;
     if (stream) cudaStreamDestroy(stream);
@@ -588,14 +587,21 @@ int alloc_staged(SopCtx* ctx) {
   const size_t n = ((size_t)ctx->s.nbead + tb - 1) / tb;
   ts.ntile = (int)n;
   ts.smem = kTileSmemMost;
-  ts.cnt = ctx->dalloc<int>(n);
-  ts.bead = ctx->dalloc<int>(n * kTileCap);
-  ts.dim = ctx->dalloc<int2>(n);
-  ts.num = ctx->dalloc<int>(ctx->s.nbead);
-  ts.rep = ctx->dalloc<unsigned short>(n * tb * 16 * kTileChunks);
-  ts.small = ctx->dalloc<float4>(n * tb * kTileSmall);
-  if (!ts.cnt || !ts.bead || !ts.dim || !ts.num || !ts.rep || !ts.small)
-    return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
+  // one allocation, in steps of 256 bytes
+  auto bytes_of = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t sizes[6] = {bytes_of(sizeof(float4) * n * tb * kTileSmall),
+                           bytes_of(sizeof(unsigned short) * n * tb * 16 * kTileChunks),
+                           bytes_of(sizeof(int) * n * kTileCap), bytes_of(sizeof(int2) * n),
+                           bytes_of(sizeof(int) * n), bytes_of(sizeof(int) * (size_t)ctx->s.nbead)};
+  char* at[7] = {ctx->dalloc<char>(std::accumulate(sizes, sizes + 6, (size_t)0))};
+  if (!at[0]) return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
+  for (int k = 0; k < 6; ++k) at[k + 1] = at[k] + sizes[k];
+  ts.small = reinterpret_cast<float4*>(at[0]);
+  ts.rep = reinterpret_cast<unsigned short*>(at[1]);
+  ts.bead = reinterpret_cast<int*>(at[2]);
+  ts.dim = reinterpret_cast<int2*>(at[3]);
+  ts.cnt = reinterpret_cast<int*>(at[4]);
+  ts.num = reinterpret_cast<int*>(at[5]);
   ts.beads = tb;
   return SOP_OK;
 }
@@ -938,11 +944,11 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
       !s.cell_scan || !s.bead_cell || !s.bead_slot || !s.sorted || !s.xs || !s.flags ||
       !ctx->w.block_sums || !ctx->e_part)
     return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
-  if (!ctx->h_out) CK(cudaMallocHost(&ctx->h_out, 16 * sizeof(double)));
-  if (!ctx->h_io) {
+  if (!ctx->h_out) {  // one allocation: each takes some 100 us
     ctx->io_bytes = ctx->served ? std::max<size_t>(kServedIoBytes, 12 * nm)
                                 : 48 * (size_t)std::min<long long>(c.max_mol_beads, kPinnedBeads);
-    CK(cudaMallocHost(&ctx->h_io, ctx->io_bytes));
+    CK(cudaMallocHost(&ctx->h_out, 16 * sizeof(double) + ctx->io_bytes));
+    ctx->h_io = reinterpret_cast<char*>(ctx->h_out + 16);
   }
   if (!ctx->served && c.max_mol_beads > kPinnedBeads) {
     int rc = state_buffer(ctx, c.max_mol_beads);
