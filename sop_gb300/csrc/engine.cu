@@ -335,8 +335,8 @@ int graph_steps(const SopCtx* ctx);
 bool staged(const SopCtx* ctx) { return ctx->tiles.beads || ctx->pair_step; }
 
 // The rows of the molecule whose beads are o .. o + n - 1 in the repulsive
-// neighbour list (r = 0) or pair list (r = 1), every entry as an index
-// relative to bead o (as stored), full row stride.
+// neighbour list (r = 0) or pair list (r = 1), in row order, every entry as an
+// index relative to bead o (as stored), full row stride.
 int read_rows(SopCtx* ctx, int r, int o, int n, std::vector<int>& rows) {
   const long long stride = ctx->s.nl_stride, len = stride * n;
   rows.assign((size_t)len, 0);
@@ -344,7 +344,8 @@ int read_rows(SopCtx* ctx, int r, int o, int n, std::vector<int>& rows) {
   std::vector<unsigned short> h((size_t)len);
   CK(cudaMemcpy(h.data(), (r == 0 ? ctx->s.nl_j : ctx->s.pl_j) + (long long)o * stride,
                 sizeof(unsigned short) * len, cudaMemcpyDeviceToHost));
-  for (size_t k = 0; k < h.size(); ++k) rows[k] = h[k];
+  for (size_t k = 0; k < h.size(); ++k)  // the stride is a multiple of 32
+    rows[k] = h[r == 0 ? k : k / 16 * 16 + pl_at((int)(k % 16))];
   return SOP_OK;
 }
 
@@ -1855,13 +1856,17 @@ int restore_into(SopCtx* ctx, int slot, const char* buf, long long len) {
   std::vector<unsigned short> rows[2];   // both molecule-relative, as stored
   for (int k = 0; k < 2; ++k) {
     rows[k].assign((size_t)(stride * n), 0);
-    for (int i = 0; i < n; ++i)
-      for (int t = 0; t < cnt[(size_t)(2 + k) * n + i]; ++t) {
+    for (int i = 0; i < n; ++i) {
+      unsigned short* row = rows[k].data() + (size_t)i * stride;
+      const int c = cnt[(size_t)(2 + k) * n + i];
+      for (int t = 0; t < c; ++t) {
         int v;
         get(&v, sizeof v);
         if (v < 0 || v >= n) return ctx->fail(SOP_ERR_ARG, "corrupt checkpoint");
-        rows[k][(size_t)i * stride + t] = (unsigned short)v;
+        row[k == 0 ? t : pl_at(t)] = (unsigned short)v;
       }
+      for (int t = c; k == 1 && (t & 15); ++t) row[pl_at(t)] = (unsigned short)i;
+    }
   }
   const int cur = (int)(h.step & 1);
   float4* dst[7] = {s.x[cur] + o, s.x[cur ^ 1] + o, s.p[cur] + o, s.p[cur ^ 1] + o,

@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, EnergyJob j
       float4 xx[kTermBatch];
 #pragma unroll
       for (int c = 0; c < kTermBatch; ++c)
-        xx[c] = X[jbase + (int)s.pl_j[rbase + min(e0 + c, rcnt - 1)]];
+        xx[c] = X[jbase + (int)s.pl_j[rbase + pl_at(min(e0 + c, rcnt - 1))]];
 #pragma unroll
       for (int c = 0; c < kTermBatch; ++c) {
         if (e0 + c >= rcnt) break;

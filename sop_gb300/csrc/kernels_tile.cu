@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_pl_tile(DevSys s, TileSet ts,
     } else {  // the rows stay as they are
       nrep = s.pl_cnt[i];
       natt = s.pl_att_cnt[i];
-      for (int e = lane; e < nrep; e += 32) mark(start + (int)s.pl_j[(long long)i * s.nl_stride + e]);
+      for (int e = lane; e < nrep; e += 32) mark(start + (int)s.pl_j[(long long)i * s.nl_stride + pl_at(e)]);
       for (int e = lane; e < natt; e += 32) mark(__float_as_int(s.pl_att[s.nat_row[i].x + e].x));
     }
     for (int e = lane; e < br.y; e += 32) mark(s.bond_j[br.x + e]);
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_pl_tile(DevSys s, TileSet ts,
     const unsigned short* row = s.pl_j + (long long)i * s.nl_stride;
     // past the row's end the partner is the bead itself (d2 = 0 contributes 0)
     for (int e = lane; e < 16 * own; e += 32)
-      rep[tile_rep_at<TB>(q, e)] = (unsigned short)(e < nrep ? local(start + (int)row[e]) : self);
+      rep[tile_rep_at<TB>(q, e)] = (unsigned short)(e < nrep ? local(start + (int)row[pl_at(e)]) : self);
     float4* out = ts.small + (long long)tile * kTileSmall * TB + q;
     for (int e = lane; e < nsmall; e += 32) {
       float4 a = make_float4(0.f, 0.f, 0.f, __int_as_float(1));  // {r0, eps, position, type}
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
 #pragma unroll
         for (int c = 0; c < kB; ++c) {
           const int e = e0 + c * G;
-          xx[c] = e < nrep ? X[start + (int)(e < kPairRep ? rrow[q][e] : grow[e])] : xi;
+          xx[c] = e < nrep ? X[start + (int)(e < kPairRep ? rrow[q][e] : grow[pl_at(e)])] : xi;
         }
 #pragma unroll
         for (int c = 0; c < kB; ++c)  // past the row's end: the bead itself contributes 0

@@ -130,10 +130,11 @@ __device__ __forceinline__ void pair_rows_w(const DevSys& s, const float4* X, in
     for (int q = 0; q < 4; ++q)
       if (pb & (1u << q)) {
         rep(pos, jq[q] - mstart);
-        out[pos++] = (unsigned short)(jq[q] - mstart);
+        out[pl_at(pos++)] = (unsigned short)(jq[q] - mstart);
       }
     k += __shfl_sync(gmask, incl, L - 1, L);
   }
+  for (int e = k + lane; e < ((k + 15) & ~15); e += L) out[pl_at(e)] = (unsigned short)irel;
   if (lane == 0) s.pl_cnt[i] = k;
   int ka = 0;
   for (int e0 = 0; e0 < acnt; e0 += L) {

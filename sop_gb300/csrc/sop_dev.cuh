@@ -19,8 +19,10 @@
 //                         65,535 beads); a row that would outgrow the stride
 //                         raises the overflow flag and the host regrows
 //   pl_cnt, pl_j    u16   repulsive pair list in the same row layout: row i
-//                         is the first pl_cnt[i] entries at i*nl_stride (an
-//                         in-order compaction of the neighbour-list row)
+//                         is pl_cnt[i] entries from i*nl_stride on (an
+//                         in-order compaction of the neighbour-list row),
+//                         entry e at pl_at(e), filled up to a whole chunk of
+//                         16 with the bead itself (which contributes 0)
 //   nl_att_cnt/nl_att_e   attractive neighbour list: native-entry indices in
 //                         the native row layout
 //   pl_att_cnt/pl_att     attractive pair list, float4 {j bits, r0, eps, 0}
@@ -31,6 +33,13 @@
 namespace sop {
 
 constexpr int kMaxLanes = 32;
+
+// Position of entry e in a repulsive pair-list row.  The force sum takes a row
+// in chunks of 16, entries l, l + 4, l + 8, l + 12 in lane l of four: as one
+// word of 8 bytes (its own inverse: the chunk is a transposed 4 x 4 square).
+__host__ __device__ __forceinline__ int pl_at(int e) {
+  return (e & ~15) | ((e & 3) << 2) | ((e >> 2) & 3);
+}
 
 // Molecules of up to this many beads are binned by one block each (12 bytes
 // of shared memory a bead); larger ones by a chain of kernels.

@@ -10,12 +10,51 @@ namespace sop {
 struct GlobalX {
   const float4* __restrict__ p;
   __device__ __forceinline__ float4 operator()(int j) const { return p[j]; }
+  __device__ __forceinline__ GlobalX from(int b) const { return {p + b}; }
 };
 struct WindowX {
   const float4* p;  // shared memory
   int off;
   __device__ __forceinline__ float4 operator()(int j) const { return p[j - off]; }
+  __device__ __forceinline__ WindowX from(int b) const { return {p, off - b}; }
 };
+
+// A lane's share of a chunk of kV = 16 entries of a repulsive pair-list row:
+// entries lane + c * G, which pl_at lays into one word (at G = 2 into two).
+// As 2-byte loads, each with its bounds test, the indexes took as many loads as
+// the coordinates; now the next chunk's word is on its way while one is summed.
+// us per 50 steps at 4 lanes, list rebuilds included: 50,000 beads 1,317 -> 1,285,
+// half of the ensemble of 512 1,886 -> 1,830 (without the read-ahead 50,000 beads
+// in one kernel 1,449 -> 1,431 against 1,475 -> 1,425).
+template <int G>
+__device__ __forceinline__ uint2 chunk_word(const uint2* __restrict__ chunk, int lane) {
+  if (G >= 16) return make_uint2(reinterpret_cast<const unsigned short*>(chunk)[pl_at(lane)], 0u);
+  return chunk[lane & 3];  // at G = 8 lanes l and l + 4 share a word
+}
+template <int G>
+__device__ __forceinline__ void chunk_partners(uint2 w, const uint2* __restrict__ chunk, int lane,
+                                               unsigned (&jj)[kV / G]) {
+  constexpr int kC = kV / G;
+  if (G >= 16) {
+    jj[0] = w.x;
+  } else if (G == 8) {  // entries l, l + 8 of the word's l, l + 4, l + 8, l + 12
+    const unsigned half = lane & 4 ? 0x4432u : 0x4410u;
+    jj[0] = __byte_perm(w.x, 0u, half);
+    jj[1 % kC] = __byte_perm(w.y, 0u, half);
+  } else {
+    jj[0] = w.x & 0xffffu;
+    jj[(4 / G) % kC] = w.x >> 16;
+    jj[(8 / G) % kC] = w.y & 0xffffu;
+    jj[(12 / G) % kC] = w.y >> 16;
+    if (G == 2) {
+      const uint2 v = chunk[lane + 2];
+      jj[1] = v.x & 0xffffu;
+      jj[3 % kC] = v.x >> 16;
+      jj[5 % kC] = v.y & 0xffffu;
+      jj[7 % kC] = v.y >> 16;
+    }
+  }
+}
 
 // The kV partial sums of a bead, kC = kV / G in each of its G lanes: upper
 // levels of the fixed tree inside the lane, lower levels by shuffles; the
@@ -70,6 +109,9 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
   const float boxl = s.boxl;
   const bool wrap = s.grid[m1].wrap != 0;
   const long long rbase = (long long)i * s.nl_stride;
+  const uint2* __restrict__ prow = reinterpret_cast<const uint2*>(s.pl_j + rbase);
+  uint2 next = make_uint2(0u, 0u);
+  if (rcnt > 0) next = chunk_word<G>(prow, lane);
 
   // Bonded, angle and native terms share one index space [bonds | angles |
   // natives]; a bead has a handful of them, usually one pass.
@@ -107,18 +149,15 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
   // Non-native repulsion, kC loads in flight per lane per chunk of kV entries
   const RepConst rc = rep_const(s);
   // pair-list partners are stored relative to the molecule's first bead
-  const unsigned short* __restrict__ prow = s.pl_j + rbase;
-  const int jbase = s.mol[m1].start;
-  for (int base = 0; base < rcnt; base += kV) {
-    int jj[kC];
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      const int e = base + lane + c * G;
-      jj[c] = e < rcnt ? jbase + (int)prow[e] : i;
-    }
+  const XS Xm = X.from(s.mol[m1].start);
+  for (int base = 0; base < rcnt; base += kV, prow += kV / 4) {
+    const uint2 w = next;
+    if (base + kV < rcnt) next = chunk_word<G>(prow + kV / 4, lane);
+    unsigned jj[kC];
+    chunk_partners<G>(w, prow, lane, jj);
     float4 xx[kC];
 #pragma unroll
-    for (int c = 0; c < kC; ++c) xx[c] = X(jj[c]);
+    for (int c = 0; c < kC; ++c) xx[c] = Xm(jj[c]);
 #pragma unroll
     for (int c = 0; c < kC; ++c) {
       // past the row end xx[c] is bead i itself: d2 = 0 fails the tolerance
