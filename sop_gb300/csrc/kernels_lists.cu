@@ -618,6 +618,8 @@ __global__ void __launch_bounds__(kNlThreads, 4) k_nl(DevSys s, int koff) {
       }
     }
   }
+  // the list filters take entries four at a time (the stride is a multiple of 4)
+  if (lane < (-cnt & 3) && cnt < stride) row[cnt + lane] = (unsigned short)(i - mstart);
   if (lane == 0) {
     s.nl_cnt[i] = cnt < stride ? cnt : (int)stride;
     if (cnt > stride) {

@@ -16,7 +16,8 @@
 //                         starts at i*nl_stride (64-byte aligned), holds
 //                         nl_cnt[i] partners, each as its index minus the
 //                         molecule's first bead (molecules hold at most
-//                         65,535 beads); a row that would outgrow the stride
+//                         65,535 beads), the last four filled up with any of
+//                         its beads; a row that would outgrow the stride
 //                         raises the overflow flag and the host regrows
 //   pl_cnt, pl_j    u16   repulsive pair list in the same row layout: row i
 //                         is pl_cnt[i] entries from i*nl_stride on (an
