@@ -561,16 +561,23 @@ int keep_last(SopCtx* ctx) {
 // step (factor cut-offs): 128 beads 389 / 570, 2,000 529 / 686, 8,000 682 / 980,
 // 16,000 833 / 1,188.
 constexpr long long kStagedBeads = 16384, kStagedSmall = 8192;
+// With short rows the second lasts as long as its blocks (8 lanes a bead, four
+// blocks an SM) run as one wave: 18,000 beads 977 -> 715 us, 20,000 extended 502
+// / 493, 24,000 1,108 / 1,097, 120 molecules of 200-450 beads 1,977 / 2,150.
+// With long ones it loses past kStagedBeads: 80 molecules of 100-1,500 beads at
+// 32 A 2,384 / 2,926.
+constexpr long long kPairBeads = 152 * 4 * 32, kPairShortRow = 512;
 int alloc_staged(SopCtx* ctx) {
   const sop_params& P = ctx->P;
   TileSet& ts = ctx->tiles;
   ts = TileSet{};
   ctx->pair_step = 0;
   const int lanes = lanes_for(ctx);
+  const bool pair = P.nplup <= 1, short_rows = ctx->s.nl_stride <= kPairShortRow;
   if (ctx->served || P.step_split > 1 || P.step_window > 0 || P.step_buckets > 0 ||
-      ctx->s.nbead > kStagedBeads)
+      ctx->s.nbead > (pair && short_rows ? kPairBeads : kStagedBeads))
     return SOP_OK;
-  if (P.nplup <= 1) {
+  if (pair) {
     if (lanes && lanes != 8 && lanes != 16) return SOP_OK;
     for (int b = 0; b < 2; ++b) {
       ctx->s.xl[b] = ctx->dalloc<float4>(ctx->s.nbead);
@@ -579,7 +586,7 @@ int alloc_staged(SopCtx* ctx) {
     // 8 lanes for larger contexts, but not for long rows (up to 512 entries at
     // the factor cut-offs, 1,088 at 32 A): us per 50 steps with 8 / 16 lanes,
     // 8,000 beads 708 / 682, 12,000 758 / 901; 10,900 beads at 32 A 1,354 / 1,096
-    const bool eight = ctx->s.nbead > kStagedSmall && ctx->s.nl_stride <= 512;
+    const bool eight = ctx->s.nbead > kStagedSmall && short_rows;
     ctx->pair_step = lanes ? lanes : eight ? 8 : 16;
     return keep_last(ctx);
   }
