@@ -66,3 +66,21 @@ def test_forces_of_rows(n, lanes, split):
         r2, s2, _ = e.list_pairs(0, 3)
         assert np.array_equal(r2, ri) and np.array_equal(s2, rj)
         assert np.array_equal(forces(e), want)
+
+
+@pytest.mark.parametrize("n", [16385, 19456, 19457])
+def test_list_and_step_in_one_launch_of_large_contexts(n):
+    """The edges of the range where short rows keep the staged form, against the
+    two-kernel form: the same bits."""
+    m, x = start(n)
+    got = []
+    for split in (1, 2):
+        e = engine.Engine(engine.default_params(h=0.05, zeta=0.05, step_split=split))
+        e.add(m, x, T=0.6)
+        e.commit()
+        e.step(13)
+        got.append([*(e.download(0)[k] for k in ("unc_pos", "vel", "force")), e.energy(0),
+                    *e.list_pairs(0, 3)])
+        e.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
