@@ -127,9 +127,8 @@ __global__ void __launch_bounds__(kThreads) k_energy_lists(Lists L, double* __re
 // Final FP64 sum of the partials (e_bnd gets -(k R0^2 / 2), energy.cu:223),
 // then rna_etot (energy.cu:76).  One block; a thread per term took 23 us at 484
 // partials, the loads one after another.
-__global__ void __launch_bounds__(kFinalThreads) k_energy_lists_final(const double* __restrict__ scratch,
-                                                                       int nblocks, double bnd_coeff,
-                                                                       double* __restrict__ out) {
+__global__ void __launch_bounds__(kFinalThreads) k_energy_lists_final(const double* scratch, int nblocks,
+                                                                       double bnd_coeff, double* out) {
   __shared__ double red[4 * 32];
   __shared__ double t[4];
   pdl_wait();

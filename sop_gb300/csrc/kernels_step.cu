@@ -227,7 +227,7 @@ __device__ __forceinline__ void tile_body(const DevSys& s, int koff, int4 t, flo
 
 template <bool STEP, bool UNI>
 __global__ void __launch_bounds__(kStepThreads, StepBlocks<4>::value)
-    k_step_tiles(DevSys s, int koff, const int4* __restrict__ tiles) {
+    k_step_tiles(DevSys s, int koff, const int4* tiles) {
   __shared__ float4 fsum[kStepThreads / 4];
   __shared__ int bead[kStepThreads / 4];
   pdl_wait();
@@ -512,11 +512,9 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, EnergyJob j
 // thread per term took 12 us at 196 partials, the loads one after another).
 constexpr int kFinalThreads = 256;
 
-__global__ void __launch_bounds__(kFinalThreads) k_energy_final(const double* __restrict__ part,
-                                                                 EnergyJob job,
-                                                                 const RetireJob* __restrict__ jobs,
-                                                                 double k_bnd_R0sq_half,
-                                                                 double* __restrict__ out) {
+__global__ void __launch_bounds__(kFinalThreads) k_energy_final(const double* part, EnergyJob job,
+                                                                 const RetireJob* jobs,
+                                                                 double k_bnd_R0sq_half, double* out) {
   __shared__ double red[4 * 32];
   pdl_wait();
   if (jobs) job = jobs[blockIdx.y].e;
@@ -580,9 +578,8 @@ __global__ void __launch_bounds__(kEnergyThreads) k_observables(DevSys s, int mo
 }
 
 // (A single thread took 55 us over 196 blocks' partials.)
-__global__ void __launch_bounds__(kFinalThreads) k_observables_final(const double* __restrict__ part,
-                                                                      int nblocks, int n, int nnat,
-                                                                      double* __restrict__ out) {
+__global__ void __launch_bounds__(kFinalThreads) k_observables_final(const double* part, int nblocks,
+                                                                      int n, int nnat, double* out) {
   __shared__ double red[8 * 32];
   __shared__ double t[8];
   pdl_wait();

@@ -162,8 +162,14 @@ enum { FLAG_NL_OVERFLOW = 1, FLAG_BARRIER_TIMEOUT = 2 };
 // scheduled while the previous kernel's last wave drains.  pdl_wait() blocks
 // until the previous kernel on the stream has completed and its writes are
 // visible (a no-op after an ordinary launch); pdl_release() lets the next
-// kernel be scheduled.  Each such kernel waits before its first global access,
-// so completion is transitive along the chain.
+// kernel be scheduled.  Every thread of such a kernel waits before it returns
+// and before it reads what an earlier kernel of the chain writes, so completion
+// is transitive along the chain.
+//
+// Nothing such a kernel reads is passed as const __restrict__: the qualifier
+// promises that the data does not change while the kernel lives, which starts
+// before the kernel that writes it has finished, and lets the compiler take
+// loads through the read-only path, which the wait does not order.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -8,7 +8,7 @@ namespace sop {
 // global memory, or the block's window of it staged in shared memory (bead j
 // at xw[j - off]).  The arithmetic is the same either way, so are the bits.
 struct GlobalX {
-  const float4* __restrict__ p;
+  const float4* p;
   __device__ __forceinline__ float4 operator()(int j) const { return p[j]; }
   __device__ __forceinline__ GlobalX from(int b) const { return {p + b}; }
 };
@@ -27,12 +27,12 @@ struct WindowX {
 // half of the ensemble of 512 1,886 -> 1,830 (without the read-ahead 50,000 beads
 // in one kernel 1,449 -> 1,431 against 1,475 -> 1,425).
 template <int G>
-__device__ __forceinline__ uint2 chunk_word(const uint2* __restrict__ chunk, int lane) {
+__device__ __forceinline__ uint2 chunk_word(const uint2* chunk, int lane) {
   if (G >= 16) return make_uint2(reinterpret_cast<const unsigned short*>(chunk)[pl_at(lane)], 0u);
   return chunk[lane & 3];  // at G = 8 lanes l and l + 4 share a word
 }
 template <int G>
-__device__ __forceinline__ void chunk_partners(uint2 w, const uint2* __restrict__ chunk, int lane,
+__device__ __forceinline__ void chunk_partners(uint2 w, const uint2* chunk, int lane,
                                                unsigned (&jj)[kV / G]) {
   constexpr int kC = kV / G;
   if (G >= 16) {
@@ -109,7 +109,7 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
   const float boxl = s.boxl;
   const bool wrap = s.grid[m1].wrap != 0;
   const long long rbase = (long long)i * s.nl_stride;
-  const uint2* __restrict__ prow = reinterpret_cast<const uint2*>(s.pl_j + rbase);
+  const uint2* prow = reinterpret_cast<const uint2*>(s.pl_j + rbase);
   uint2 next = make_uint2(0u, 0u);
   if (rcnt > 0) next = chunk_word<G>(prow, lane);
 
