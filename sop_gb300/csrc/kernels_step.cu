@@ -167,21 +167,26 @@ __global__ void __launch_bounds__(kStepThreads, StepBlocks<G>::value) k_step(Dev
 template <bool STEP>
 __global__ void __launch_bounds__(256, 6) k_finish(DevSys s, int koff) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= s.nlive) return;
-  const int m = s.mol_of[b];
-  if (m < 0) return;  // a free slot: nothing was summed
+  const int m = b < s.nlive ? s.mol_of[b] : -1;  // -1: a free slot, nothing was summed
   // a molecule k_step skips for good (inactive, not started or finished:
   // the tests of bead_slot on values no kernel of this step writes) has
   // nothing to finish; a stopped one is caught by its unmarked sum below
   // (its status bits may be set by this very kernel)
-  const MolConst& mc = s.mol[m];
-  const long long n = s.mol_step[m] + (STEP ? 1 : 0) + koff;
-  if (!mc.active || n < 0 || (STEP && mc.nsteps >= 0 && n > mc.nsteps)) return;
-  const int cur = (int)(n & 1);
+  bool due = false;
+  int cur = 0;
   BeadState t;
-  load_bead_state<STEP>(s, b, m, koff, cur, t);
+  if (m >= 0) {
+    const MolConst& mc = s.mol[m];
+    const long long n = s.mol_step[m] + (STEP ? 1 : 0) + koff;
+    due = mc.active && n >= 0 && !(STEP && mc.nsteps >= 0 && n > mc.nsteps);
+    cur = (int)(n & 1);
+    if (due) load_bead_state<STEP>(s, b, m, koff, cur, t);
+  }
+  // every thread: a grid of which all returned here would have completed
+  // before the force kernel it follows, and what comes next with it
   pdl_wait();
   pdl_release();
+  if (!due) return;
   const float4 fs = s.fsum[b];
   if (__float_as_int(fs.w) == 0) return;  // not summed this step
   s.fsum[b].w = 0.0f;

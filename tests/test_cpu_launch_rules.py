@@ -1,6 +1,7 @@
 """Rules of programmatic dependent launch that the compiler does not check, read
 from the kernels' source: a kernel that waits for its predecessor
-(griddepcontrol.wait, pdl_wait()) takes no data as const __restrict__."""
+(griddepcontrol.wait, pdl_wait()) takes no data as const __restrict__, and no
+thread of it returns before it has waited."""
 import os
 import re
 
@@ -52,3 +53,11 @@ def test_waiting_kernels_take_nothing_as_const_restrict(f, name, params):
 @pytest.mark.parametrize("f", ["step_force.cuh", "step_dev.cuh", "lists_dev.cuh", "kernels_tile.cu"])
 def test_code_of_waiting_kernels_reads_nothing_as_const_restrict(f):
     assert not re.search(r"const[\w\s]*\*\s*__restrict__", source(f))
+
+
+@pytest.mark.parametrize("f,name,body", [(w[0], w[1], w[3]) for w in WAITING],
+                         ids=[w[1] for w in WAITING])
+def test_no_thread_returns_before_the_wait(f, name, body):
+    """A grid all of whose threads returned first would complete before the
+    kernel it follows, and the kernels after it would not wait for that one."""
+    assert not re.search(r"\breturn\b", body[:body.index("pdl_wait()")]), (f, name)
