@@ -34,7 +34,6 @@ struct NLScratch {
 };
 void launch_nl_rebuild(const DevSys& s, const NLScratch& w, int koff, cudaStream_t st);
 void launch_pl_rebuild(const DevSys& s, int koff, cudaStream_t st);
-void launch_rebin(const DevSys& s, const NLScratch& w, cudaStream_t st);
 void launch_scan(const int* in, long long n, int* out, int* block_sums, cudaStream_t st);
 long long scan_block_sums_needed(long long n);
 // kernels_step.cu
@@ -1893,6 +1892,12 @@ int restore_into(SopCtx* ctx, int slot, const char* buf, long long len) {
                 sizeof(unsigned short) * rows[1].size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(s.mol_step + slot, &h.step, sizeof(long long), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(s.mol_status + slot, &h.status, sizeof(int), cudaMemcpyHostToDevice));
+  // The lists may hold pairs through the molecule's image that its restored
+  // coordinates no longer show, so the minimum image is applied until the next
+  // neighbour-list rebuild, where it is the identity too.
+  MolGrid g{};
+  g.wrap = g.wrap_list = 1;
+  CK(cudaMemcpy(s.grid + slot, &g, sizeof g, cudaMemcpyHostToDevice));
   return SOP_OK;
 }
 
@@ -1957,7 +1962,6 @@ static int serve_round(SopCtx* ctx) {
   // admission in arrival order; a job that does not fit yet lets the next
   // few (smaller) ones try
   int looked = 0;
-  bool rebin = false;
   Arrivals arrivals;
   for (auto it = ctx->queue.begin(); it != ctx->queue.end() && looked < 64 && !ctx->free_slots.empty();) {
     Job& jb = ctx->jobs[*it];
@@ -1980,13 +1984,11 @@ static int serve_round(SopCtx* ctx) {
     }
     if (rc) return rc;
     if (resumed) {
-      // the job continues at its checkpoint's step: its state and lists come
-      // from the checkpoint, and the binning below sets the molecule's grid flags
+      // the job continues at its checkpoint's step, with its state and lists
       rc = restore_into(ctx, slot, jb.resume.data(), (long long)jb.resume.size());
       if (rc) return rc;
       jb.resume.clear();
       jb.resume.shrink_to_fit();
-      rebin = true;
     }
     ctx->free_slots.pop_back();
     ctx->slot_job[slot] = *it;
@@ -1997,10 +1999,6 @@ static int serve_round(SopCtx* ctx) {
   rc = flush_arrivals(ctx, arrivals);
   if (rc) return rc;
   update_live(ctx);
-  if (rebin) {
-    launch_rebin(ctx->s, ctx->w, ctx->stream);
-    CK(cudaGetLastError());
-  }
   bool any = false;
   for (int id : ctx->slot_job) any |= id >= 0;
   if (any) return step_async(ctx, ctx->P.nnlup);
@@ -2610,9 +2608,6 @@ int sop_restore(void* p, int mol, const void* buf, long long size) {
     return ctx->fail(SOP_ERR_ARG, "checkpoint step differs from the context's step");
   rc = restore_into(ctx, mol, static_cast<const char*>(buf), size);
   if (rc) return rc;
-  // refresh each molecule's grid flags (and the cell order) from the restored
-  // coordinates: binning only, no list changes
-  launch_rebin(ctx->s, ctx->w, ctx->stream);
   if (ctx->tiles.beads) CK(launch_pl_tile(ctx->s, ctx->tiles, 0, true, ctx->stream));
   rc = keep_last(ctx);
   if (rc) return rc;

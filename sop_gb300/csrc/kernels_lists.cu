@@ -713,14 +713,6 @@ void launch_nl_rebuild(const DevSys& s, const NLScratch& w, int koff, cudaStream
   }
 }
 
-// The binning alone, every list untouched: molecules that arrive with their
-// lists (restored from a checkpoint) get grid flags from their own
-// coordinates, which the step and pair-list kernels need.  The cell order
-// itself decides no result.
-void launch_rebin(const DevSys& s, const NLScratch& w, cudaStream_t st) {
-  launch_binning(s, w, 0, st);
-}
-
 void launch_pl_rebuild(const DevSys& s, int koff, cudaStream_t st) {
   const int T = 256;
   const int L = s.nlive <= kWideListBeads ? 32 : (s.long_rows ? 16 : 8);
