@@ -504,13 +504,14 @@ int wait_flags(SopCtx* ctx, int* flags) {
 
 // Neighbour-list rebuild, and what `then` queues behind it, that regrows the
 // rows on overflow and runs again; only_mol >= 0 rebuilds that molecule's
-// lists alone.  Synchronous.
+// lists alone; keep_wrap: no pair-list rebuild follows.  Synchronous.
 template <class F>
-int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol, F then) {
+int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol, bool keep_wrap, F then) {
   ctx->queued = true;
   for (int attempt = 0; attempt < 4; ++attempt) {
     DevSys s = ctx->s;  // re-read: a regrow changes the rows
     s.only_mol = only_mol;
+    s.keep_wrap = keep_wrap ? 1 : 0;
     launch_nl_rebuild(s, ctx->w, koff, ctx->stream);
     int rc = then(s);
     if (rc) return rc;
@@ -527,8 +528,8 @@ int nl_rebuild_checked(SopCtx* ctx, int koff, int only_mol, F then) {
   }
   return ctx->fail(SOP_ERR_CAPACITY, "neighbour list kept overflowing");
 }
-int nl_rebuild_checked(SopCtx* ctx, int koff) {
-  return nl_rebuild_checked(ctx, koff, -1, [](const DevSys&) { return (int)SOP_OK; });
+int nl_rebuild_checked(SopCtx* ctx, int koff, bool keep_wrap = false) {
+  return nl_rebuild_checked(ctx, koff, -1, keep_wrap, [](const DevSys&) { return (int)SOP_OK; });
 }
 
 // Pair-list rebuild of the molecules of s, and of the tables the tile step
@@ -2194,7 +2195,7 @@ int sop_upload_state(void* p, int mol, const float* pos, const float* unc_pos, c
   launch_unpack_state(ctx->s, hm.start, hm.n, in[0] ? in[0] : in[1], in[1], in[2], ctx->stream);
   // the lists of this molecule alone: the others keep theirs (built from
   // their own step's coordinates; buffer step - 1 holds their look-ahead)
-  return nl_rebuild_checked(ctx, -1, mol, [&](const DevSys& one) {
+  return nl_rebuild_checked(ctx, -1, mol, false, [&](const DevSys& one) {
     int e = keep_last(ctx);
     if (e) return e;
     rebuild_pairs(ctx, one, -1);
@@ -2241,7 +2242,12 @@ int sop_launch_stage(void* p, int stage, int koff) {
       else launch_steps(ctx, koff, 1);
       break;
     case 1: rebuild_pairs(ctx, ctx->s, koff); break;
-    case 2: launch_nl_rebuild(ctx->s, ctx->w, koff, ctx->stream); break;
+    case 2: {
+      DevSys s = ctx->s;
+      s.keep_wrap = 1;
+      launch_nl_rebuild(s, ctx->w, koff, ctx->stream);
+      break;
+    }
     case 3: launch_advance(ctx->s, koff, ctx->stream); break;
     default: return ctx->fail(SOP_ERR_ARG, "unknown stage");
   }
@@ -2255,7 +2261,7 @@ int sop_update_neighbor_list(void* p, long long* nnl_att, long long* nnl_rep) {
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
-  rc = nl_rebuild_checked(ctx, 0);
+  rc = nl_rebuild_checked(ctx, 0, true);
   if (rc) return rc;
   if (nnl_att || nnl_rep) {
     std::vector<int> a(ctx->s.nbead), r(ctx->s.nbead);

@@ -157,8 +157,9 @@ __global__ void k_bbox(DevSys s, int koff) {
 }
 
 // The cell grid of a molecule of n beads within the bounds b (ordered floats:
-// three lower, three upper).
-__device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsigned* b, int base) {
+// three lower, three upper); old: its grid so far.
+__device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsigned* b, int base,
+                                             const MolGrid& old) {
   MolGrid g = {};
   float lo[3], ext[3];
   for (int a = 0; a < 3; ++a) {
@@ -218,6 +219,10 @@ __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsig
   // their separations stay below boxl/2 however far the molecule reaches (a
   // 50,000-bead globule, 340 A across, in a box of 500 A).
   g.wrap_list = wrap && (g.brute || s.wrap_from < 0.5f || !(4.1f * rc < s.boxl)) ? 1 : 0;
+  if (s.keep_wrap) {  // its pair list stays, and may hold pairs through the image
+    g.wrap |= old.wrap;
+    g.wrap_list |= old.wrap_list;
+  }
   g.ncell = g.dims[0] * g.dims[1] * g.dims[2];
   g.base = base;
   return g;
@@ -304,7 +309,7 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
       }
       __syncthreads();
       if (t == 0) {
-        grid = make_grid(s, n, bounds, cell_base(start));
+        grid = make_grid(s, n, bounds, cell_base(start), s.grid[m]);
         s.grid[m] = grid;
       }
       __syncthreads();
@@ -359,7 +364,7 @@ __global__ void k_grid(DevSys s, int koff) {
   if (m >= s.nmol || !bins_by_chain(s, m, koff)) return;
   unsigned b[6];
   for (int a = 0; a < 6; ++a) b[a] = s.bbox[6 * m + a];
-  s.grid[m] = make_grid(s, s.mol[m].n, b, cell_base(s.mol[m].start));
+  s.grid[m] = make_grid(s, s.mol[m].n, b, cell_base(s.mol[m].start), s.grid[m]);
 }
 
 __global__ void k_assign(DevSys s, int koff) {

@@ -74,6 +74,7 @@ struct DevSys {
   int nbead, nmol;
   int nlive;                    // bead slots the per-step kernels cover; every slot past it is free
   int only_mol;                 // >= 0: a list rebuild covers this molecule alone (a state upload)
+  int keep_wrap;                // 1: a neighbour-list rebuild that no pair-list rebuild follows
   float boxl;
   float eps_rep;
   int rep6;

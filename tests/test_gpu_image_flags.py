@@ -110,3 +110,22 @@ def test_restore_of_one_molecule_leaves_the_other(kw):
     e.close()
     for a, b in zip(got, want):
         same(a, b)
+
+
+@pytest.mark.parametrize("kw", [FORMS[0], FORMS[2], FORMS[3]])
+@pytest.mark.parametrize("how", ["update", "stage"])
+def test_neighbour_list_by_the_caller_keeps_the_pair_list_s_image(how, kw):
+    """The caller's own neighbour-list rebuild between two pair-list rebuilds:
+    the steps until the next one sum the same pairs, so the same bits."""
+    want, _ = uninterrupted(**kw)
+    e, _ = context(**kw)
+    e.step(6)
+    if how == "update":
+        e.update_neighbor_list()
+    else:
+        e.launch_stage(2, 0)
+    got = state(e)
+    same(got, want[0])
+    e.step(3)
+    same(state(e), want[1])
+    e.close()
