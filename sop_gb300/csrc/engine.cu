@@ -858,9 +858,9 @@ void set_constants(SopCtx* ctx) {
       if (a > 0 && b > 0) rcmax = std::max(rcmax, rcut_of(P.nl_rep_fac, P.nl_rep_abs, sg));
     }
   s.rc_nl_rep_max = rcmax;
-  // lists rebuilt rarely or never let pairs drift further before the next look
-  // at the extent: there the flag keeps twice the margin
-  s.wrap_from = P.nnlup > 0 && P.nnlup <= 200 ? 0.5f : 0.25f;
+  // two beads, nnlup steps and the look-ahead at either end; a tenth for rounding
+  s.move_share = P.nnlup > 0 && P.nnlup < 1 << 29 ? (float)(0.9 / (2.0 * ((double)P.nnlup + 2.0))) : 0.0f;
+  s.move_least = 0.99f * s.move_share * rcmax;  // the room is a cut-off at least (make_grid)
   s.seed_lo = (unsigned)(P.seed & 0xffffffffULL);
   s.seed_hi = (unsigned)(P.seed >> 32);
 }
@@ -923,7 +923,7 @@ int alloc_pools(SopCtx* ctx, const Caps& c) {
   s.pl_j = nullptr;
   int rc = alloc_nl(ctx, c.stride);
   if (rc) return rc;
-  s.bbox = ctx->dalloc<unsigned>(6 * nm);
+  s.bbox = ctx->dalloc<unsigned>(7 * nm);
   s.grid = ctx->dalloc<MolGrid>(nm);
   s.cell_cap = c.cells;
   s.cell_start = ctx->dalloc<int>(c.cells + 1);
@@ -1897,7 +1897,8 @@ int restore_into(SopCtx* ctx, int slot, const char* buf, long long len) {
   // coordinates no longer show, so the minimum image is applied until the next
   // neighbour-list rebuild, where it is the identity too.
   MolGrid g{};
-  g.wrap = g.wrap_list = 1;
+  g.wrap = g.wrap_list = kImageTaken;
+  g.move = INFINITY;
   CK(cudaMemcpy(s.grid + slot, &g, sizeof g, cudaMemcpyHostToDevice));
   return SOP_OK;
 }

@@ -126,9 +126,16 @@ __device__ __forceinline__ bool bins_by_chain(const DevSys& s, int m, int koff) 
 __global__ void k_bbox_reset(DevSys s) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= s.nmol) return;
-  unsigned* b = s.bbox + 6 * m;
+  unsigned* b = s.bbox + 7 * m;
   b[0] = b[1] = b[2] = f2ord(INFINITY);
   b[3] = b[4] = b[5] = f2ord(-INFINITY);
+  b[6] = f2ord(0.0f);
+}
+
+// The furthest a coordinate of bead i moved in its last look-ahead.
+__device__ __forceinline__ float last_move(const DevSys& s, int i) {
+  const float4 d = s.incr[i];
+  return fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
 }
 
 __global__ void k_bbox(DevSys s, int koff) {
@@ -139,6 +146,7 @@ __global__ void k_bbox(DevSys s, int koff) {
   if (!ok) return;
   float4 x = xbuf(s, m, koff)[i];
   unsigned peers = __match_any_sync(act, m);
+  const unsigned moved = __reduce_max_sync(peers, f2ord(last_move(s, i)));
   unsigned lo[3] = {f2ord(x.x), f2ord(x.y), f2ord(x.z)};
   unsigned mn[3], mx[3];
 #pragma unroll
@@ -147,17 +155,18 @@ __global__ void k_bbox(DevSys s, int koff) {
     mx[a] = __reduce_max_sync(peers, lo[a]);
   }
   if ((threadIdx.x & 31) == __ffs(peers) - 1) {
-    unsigned* b = s.bbox + 6 * m;
+    unsigned* b = s.bbox + 7 * m;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       atomicMin(b + a, mn[a]);
       atomicMax(b + 3 + a, mx[a]);
     }
+    atomicMax(b + 6, moved);
   }
 }
 
 // The cell grid of a molecule of n beads within the bounds b (ordered floats:
-// three lower, three upper); old: its grid so far.
+// three lower, three upper, the furthest last move); old: its grid so far.
 __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsigned* b, int base,
                                              const MolGrid& old) {
   MolGrid g = {};
@@ -171,10 +180,11 @@ __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsig
   for (int a = 0; a < 3; ++a) periodic |= !(ext[a] + rc < s.boxl);  // also true for NaN extents
   // Separations inside the box [lo, lo + ext] never exceed ext (rounding is
   // monotone), and below boxl/2 the minimum image leaves them unchanged
-  // (rint(d / boxl) is 0).  The margin of one cut-off covers the drift until the
-  // next rebuild, for the steps and pair-list filters that use the same flag.
-  bool wrap = false;
-  for (int a = 0; a < 3; ++a) wrap |= !(ext[a] + rc < s.wrap_from * s.boxl);
+  // (rint(d / boxl) is 0).  The steps and pair-list filters until the next
+  // rebuild use the same flag, so the room to boxl/2, a cut-off at least, is
+  // shared out over them as g.move.
+  bool wrap = !(s.move_share > 0.0f);  // never rebuilt: always
+  for (int a = 0; a < 3; ++a) wrap |= !(ext[a] + rc < 0.5f * s.boxl);
   if (periodic || n <= 96) {
     g.brute = 1;
   } else {
@@ -213,15 +223,20 @@ __device__ __forceinline__ MolGrid make_grid(const DevSys& s, int n, const unsig
     g.cs = 0.0f;
     g.lo[0] = g.lo[1] = g.lo[2] = 0.0f;
   }
-  g.wrap = wrap ? 1 : 0;
   // A molecule that cannot come within a cut-off of its own image is binned by
   // plain separations, and lists pairs within a cut-off of each other only:
   // their separations stay below boxl/2 however far the molecule reaches (a
   // 50,000-bead globule, 340 A across, in a box of 500 A).
-  g.wrap_list = wrap && (g.brute || s.wrap_from < 0.5f || !(4.1f * rc < s.boxl)) ? 1 : 0;
+  const bool wrap_list = wrap && (g.brute || !(s.move_share > 0.0f) || !(4.1f * rc < s.boxl));
+  g.wrap = wrap ? kImageTaken : 0;
+  g.wrap_list = wrap_list ? kImageTaken : 0;
+  g.move = wrap_list ? INFINITY
+                     : s.move_share * (0.5f * s.boxl - (wrap ? rc : fmaxf(ext[0], fmaxf(ext[1], ext[2]))));
+  // the step that follows reads coordinates one look-ahead past these
+  if (!(ord2f(b[6]) <= g.move)) g.wrap = g.wrap_list = kImageTaken;
   if (s.keep_wrap) {  // its pair list stays, and may hold pairs through the image
-    g.wrap |= old.wrap;
-    g.wrap_list |= old.wrap_list;
+    if (old.wrap) g.wrap = kImageTaken;
+    if (old.wrap_list) g.wrap_list = kImageTaken;
   }
   g.ncell = g.dims[0] * g.dims[1] * g.dims[2];
   g.base = base;
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
   extern __shared__ int bin_smem[];
   int* first = bin_smem;                                // cells: counts, then first position
   int* order = bin_smem + 2 * most + 1;        // beads in cell order
-  __shared__ unsigned bounds[6];
+  __shared__ unsigned bounds[7];
   __shared__ MolGrid grid;
   __shared__ int found[1024];
   __shared__ int nfound;
@@ -278,9 +293,10 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
       const int m = found[f];
       const int n = s.mol[m].n, start = s.mol[m].start;
       const float4* X = xbuf(s, m, koff) + start;
-      if (t < 6) bounds[t] = t < 3 ? f2ord(INFINITY) : f2ord(-INFINITY);
+      if (t < 7) bounds[t] = f2ord(t < 3 ? INFINITY : t < 6 ? -INFINITY : 0.0f);
       __syncthreads();
       unsigned mn[3], mx[3];
+      float far = 0.0f;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         mn[a] = f2ord(INFINITY);
@@ -294,7 +310,9 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
           mn[a] = min(mn[a], o[a]);
           mx[a] = max(mx[a], o[a]);
         }
+        far = fmaxf(far, last_move(s, start + r));
       }
+      const unsigned moved = __reduce_max_sync(0xffffffffu, f2ord(far));
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
@@ -306,6 +324,7 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
           atomicMin(bounds + a, mn[a]);
           atomicMax(bounds + 3 + a, mx[a]);
         }
+        atomicMax(bounds + 6, moved);
       }
       __syncthreads();
       if (t == 0) {
@@ -362,8 +381,8 @@ __global__ void __launch_bounds__(1024) k_bin_mol(DevSys s, int koff, int most) 
 __global__ void k_grid(DevSys s, int koff) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= s.nmol || !bins_by_chain(s, m, koff)) return;
-  unsigned b[6];
-  for (int a = 0; a < 6; ++a) b[a] = s.bbox[6 * m + a];
+  unsigned b[7];
+  for (int a = 0; a < 7; ++a) b[a] = s.bbox[7 * m + a];
   s.grid[m] = make_grid(s, s.mol[m].n, b, cell_base(s.mol[m].start), s.grid[m]);
 }
 

@@ -131,10 +131,10 @@ __global__ void __launch_bounds__(kStepThreads, StepBlocks<G>::value) k_step(Dev
   bool fene_bad = false;
   if (i >= 0) {  // uniform over the lane group
     if (WIN && win_n >= 0) {
-      bead_force<G, UNI>(s, WindowX{xwin, win_lo}, i, m1, lane, q.br, q.ar, q.abase, q.acnt,
+      bead_force<G, UNI>(s, WindowX{xwin, win_lo}, i, m1, n, lane, q.br, q.ar, q.abase, q.acnt,
                          q.rcnt, fx, fy, fz, fene_bad);
     } else {
-      bead_force<G, UNI>(s, GlobalX{s.x[(int)(n & 1)]}, i, m1, lane, q.br, q.ar, q.abase, q.acnt,
+      bead_force<G, UNI>(s, GlobalX{s.x[(int)(n & 1)]}, i, m1, n, lane, q.br, q.ar, q.abase, q.acnt,
                          q.rcnt, fx, fy, fz, fene_bad);
     }
   }
@@ -213,7 +213,7 @@ __device__ __forceinline__ void tile_body(const DevSys& s, int koff, int4 t, flo
   float fx = 0.f, fy = 0.f, fz = 0.f;
   bool fene_bad = false;
   if (q.i >= 0)
-    bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, lane, q.br, q.ar, q.abase,
+    bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, q.n, lane, q.br, q.ar, q.abase,
                        q.acnt, q.rcnt, fx, fy, fz, fene_bad);
   const float4 sum = marked_sum(fx, fy, fz, fene_bad, q.n);
   if (t.w) {
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kStepThreads, StepBlocks<G>::value)
       float fx = 0.f, fy = 0.f, fz = 0.f;
       bool fene_bad = false;
       if (q.i >= 0)
-        bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, lane, q.br, q.ar, q.abase,
+        bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, q.n, lane, q.br, q.ar, q.abase,
                            q.acnt, q.rcnt, fx, fy, fz, fene_bad);
       if (lane == 0) {
         fsum[slot] = marked_sum(fx, fy, fz, fene_bad, q.n);
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kBlockFormThreads, 1) k_step_block(DevSys s, i
       float fx = 0.f, fy = 0.f, fz = 0.f;
       bool fene_bad = false;
       if (q.i >= 0)
-        bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, lane, q.br, q.ar, q.abase,
+        bead_force<G, UNI>(s, GlobalX{s.x[(int)(q.n & 1)]}, q.i, q.m1, q.n, lane, q.br, q.ar, q.abase,
                            q.acnt, q.rcnt, fx, fy, fz, fene_bad);
       if (lane == 0) {
         fsum[slot] = marked_sum(fx, fy, fz, fene_bad, q.n);

@@ -272,8 +272,6 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
     const MolConst& mc = s.mol[m];
     n = s.mol_step[m] + 1 + koff;
     run = mc.active && n >= 0 && !(mc.nsteps >= 0 && n > mc.nsteps) && !frozen;
-    wrap = s.grid[m].wrap != 0;
-    wrap_list = s.grid[m].wrap_list != 0;
   }
   // a listed bead's coordinates at its own molecule's step
   auto source = [&](int b) {
@@ -302,7 +300,11 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
   }
   if (early) pdl_wait();
   pdl_release();
-  if (run) run = s.mol_status[m] == 0;
+  if (run) {  // a step may set these
+    run = s.mol_status[m] == 0;
+    wrap = s.grid[m].wrap != 0;
+    wrap_list = list_image_taken(s, m, n);
+  }
   if (t < nb) {
     const long long n2 = s.mol_step[m2] + 1 + koff;
     copy16(inc0 + t, s.incr + b0 + t);
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
     } else {
       const int i = b0 + q;
       const int2 br = s.bond_row[i], ar = s.ang_row[i];
-      bead_force<G, UNI>(s, GlobalX{s.x[(int)(n & 1)]}, i, m, lane, br, ar, s.nat_row[i].x,
+      bead_force<G, UNI>(s, GlobalX{s.x[(int)(n & 1)]}, i, m, n, lane, br, ar, s.nat_row[i].x,
                          s.pl_att_cnt[i], s.pl_cnt[i], fx, fy, fz, bad);
     }
   }
@@ -407,7 +409,11 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_pair_step(DevSys s, int kof
       copy16(dyn + win + l, s.xl[par ^ 1] + lo + l);
       copy16(dyn + l, s.x[par] + lo + l);
     }
-  if (run) run = s.mol_status[m] == 0;
+  if (run) {  // a step may set these
+    run = s.mol_status[m] == 0;
+    head.wrap = s.grid[m].wrap != 0;
+    head.wrap_list = list_image_taken(s, m, n);
+  }
   if (t < nb) {
     const int cur = (int)((s.mol_step[m2] + 1 + koff) & 1);
     copy16(inc0 + t, s.incr + b0 + t);

@@ -51,7 +51,7 @@ __device__ __forceinline__ unsigned group_mask(int wl) {
 struct PairHead {
   int cnt, acnt, mstart;
   int2 row;     // the bead's native row
-  bool wrap, wrap_list;  // from the neighbour-list build, with a cut-off of margin
+  bool wrap, wrap_list;  // the minimum image is taken (MolGrid)
   uint2 j;      // four entries of the repulsive row
   int natj;     // one of the attractive row: partner, squared cut-off, parameters
   float rc2;
@@ -65,8 +65,9 @@ __device__ __forceinline__ PairHead pair_head(const DevSys& s, int i, int m) {
   h.acnt = s.nl_att_cnt[i];
   h.row = s.nat_row[i];
   h.mstart = s.mol[m].start;
-  h.wrap = s.grid[m].wrap != 0;
-  h.wrap_list = s.grid[m].wrap_list != 0;
+  // steps write these too: not ahead of a wait, where whoever calls sets them
+  h.wrap = !kAhead && s.grid[m].wrap != 0;
+  h.wrap_list = !kAhead && s.grid[m].wrap_list != 0;
   h.j = make_uint2(0, 0);
   if (4 * lane < h.cnt) h.j = reinterpret_cast<const uint2*>(s.nl_j + (long long)i * s.nl_stride)[lane];
   h.natj = 0;

@@ -66,15 +66,22 @@ struct MolGrid {
   int base;                     // first cell
   int ncell;
   int brute;                    // 1: index-chunked cells, all pairs scanned
-  int wrap;                     // 0: no pair of the molecule can reach boxl/2 (no minimum image)
-  int wrap_list;                // 0: no pair of its repulsive lists can
+  // Whether the minimum image is taken of any pair of the molecule, and of its
+  // repulsive lists' pairs: 0 where none of them can reach boxl/2, else
+  // kImageTaken, or the mark of the step after which it is (complete_bead: a bead
+  // moved further than `move`, up to which a 0 holds until the next rebuild).
+  int wrap, wrap_list;
+  float move;
 };
+constexpr int kImageTaken = 1;
+// (Marks live for less than 2^30 steps: where lists are rebuilt more rarely there
+// are none.)
+__device__ __forceinline__ int image_mark(long long n) { return 2 + (int)(n & 0x3fffffff); }
 
 struct DevSys {
   int nbead, nmol;
   int nlive;                    // bead slots the per-step kernels cover; every slot past it is free
   int only_mol;                 // >= 0: a list rebuild covers this molecule alone (a state upload)
-  int keep_wrap;                // 1: a neighbour-list rebuild that no pair-list rebuild follows
   float boxl;
   float eps_rep;
   int rep6;
@@ -84,7 +91,7 @@ struct DevSys {
   float rc2_nl_rep[3][3];       // squared cut-offs by type pair
   float rc2_pl_rep[3][3];
   float rc_nl_rep_max;          // max neighbour-list cut-off (A)
-  float wrap_from;              // fraction of boxl a separation stays below where the minimum image is left out
+  float move_share;             // MolGrid::move as a share of the room to boxl/2
   float sig2[3][3];             // sigma_rep^2 by type pair
   float rep_tol[3][3];          // sigma_rep * 1e-7: pairs with d^2 <= this are skipped (energy.cu:555-558)
   int uniform_type;             // 1: every bead has type 1 (one sigma for all pairs)
@@ -122,7 +129,7 @@ struct DevSys {
   unsigned short* pl_j;         // repulsive PL rows, the same layout
 
   // neighbour-list build scratch
-  unsigned* bbox;               // 6 per molecule, order-preserving float bits
+  unsigned* bbox;               // 7 per molecule, order-preserving float bits (k_bbox)
   MolGrid* grid;
   int* cell_start;              // first staged bead of each cell (molecules binned by one block)
   int* cell_cnt; int* cell_scan;  // counts and their scan (larger molecules)
@@ -131,7 +138,21 @@ struct DevSys {
   int* flags;                   // bit 0: neighbour-list overflow
   float4* noise;                // injected normals or nullptr
   int use_noise;
+  int keep_wrap;                // 1: a neighbour-list rebuild that no pair-list rebuild follows
+  float move_least;             // below MolGrid::move of every molecule
 };
+
+// MolGrid::wrap_list of molecule m for the lanes that sum a bead's step n and
+// branch on it together.  The mark of step n itself, which its blocks set while
+// others read, does not count yet, so all lanes see the same.  (MolGrid::wrap,
+// on which no lanes part, is read as it is: at the coordinates of step n both ways
+// give the same bits.  us per 50 steps of the ensemble of 512 / of 50,000 beads with
+// wrap_list read as it is 3,147 / 1,313, this way 3,146 / 1,317, both by their marks
+// 3,219 / 1,350, one vote of the lanes 3,306 / 1,386.)
+__device__ __forceinline__ bool list_image_taken(const DevSys& s, int m, long long n) {
+  const int flag = s.grid[m].wrap_list;
+  return flag != 0 && flag != image_mark(n);
+}
 
 // Tables of the tile step (kernels_tile.cu), rebuilt after every pair-list
 // rebuild; a tile is `beads` consecutive bead slots.

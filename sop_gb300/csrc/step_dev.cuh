@@ -76,8 +76,8 @@ __device__ __forceinline__ float small_coeff(const DevSys& s, int type, float dx
 // One non-native repulsion (energy.cu:536-581): co1 = -6 eps / d^2 (2 (s/r)^12 +
 // (s/r)^6) [rep6: -6 eps / d^2 (s/r)^6]; pairs with d^2 <= 1e-7 sigma are
 // skipped.  A system of one bead type (UNI) uses its sigma as a constant.
-// wrap is false when no listed pair of the molecule can reach boxl/2 (from its
-// last binning, with a cut-off of margin): the minimum image is the identity.
+// wrap is false when no listed pair of the molecule can reach boxl/2 (MolGrid):
+// the minimum image is the identity.
 // (As a run-time test of every entry it cost 18% of the step's instructions
 // at 4 lanes per bead.)
 struct RepConst {
@@ -189,6 +189,13 @@ __device__ __forceinline__ void complete_bead(const DevSys& s, int b, int m, flo
   inc = make_float4(__fmaf_rn(mc.a1, vi.x, __fmul_rn(mc.a2, fxx)),
                     __fmaf_rn(mc.a1, vi.y, __fmul_rn(mc.a2, fyy)),
                     __fmaf_rn(mc.a1, vi.z, __fmul_rn(mc.a2, fzz)), 0.f);
+  // moved too far for the minimum image to stay left out until the next look at
+  // the molecule's extent
+  const float far = fmaxf(fmaxf(fabsf(inc.x), fabsf(inc.y)), fabsf(inc.z));
+  if (!(far <= s.move_least) && !(far <= s.grid[m].move)) {
+    if (!s.grid[m].wrap) s.grid[m].wrap = image_mark(t.nb);
+    if (!s.grid[m].wrap_list) s.grid[m].wrap_list = image_mark(t.nb);
+  }
   s.incr[b] = inc;
   s.x[cur ^ 1][b] = make_float4(__fadd_rn(xo.x, inc.x), __fadd_rn(xo.y, inc.y),
                                 __fadd_rn(xo.z, inc.z), xo.w);

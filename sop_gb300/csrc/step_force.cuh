@@ -88,7 +88,7 @@ __device__ __forceinline__ void group_sum(float (&ax)[kV / G], float (&ay)[kV / 
   fz = az[0];
 }
 
-// The conservative force on bead i, summed by the G lanes of its group over
+// The conservative force on bead i at step n's coordinates, summed by the G lanes of its group over
 // its rows (bonds, angles, native pair list, repulsive pair list) into the
 // lane's kC virtual-lane accumulators, reduced to lane 0 of the group.
 // Forces are summed in a fixed order whatever G is: entry e of a row
@@ -98,8 +98,8 @@ __device__ __forceinline__ void group_sum(float (&ax)[kV / G], float (&ay)[kV / 
 // upper tree levels locally, the rest by shuffles.  So every G gives
 // bit-identical forces, and G is free to tune per context.
 template <int G, bool UNI, bool wrap_list, class XS>
-__device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i, int m1, int lane,
-                                           int2 br, int2 ar, int abase, int acnt, int rcnt,
+__device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i, int m1, long long n,
+                                           int lane, int2 br, int2 ar, int abase, int acnt, int rcnt,
                                            float& fx, float& fy, float& fz, bool& fene_bad) {
   constexpr int kC = kV / G;
   float ax[kC], ay[kC], az[kC];
@@ -171,13 +171,13 @@ __device__ __forceinline__ void bead_force_w(const DevSys& s, const XS& X, int i
 // Compiled with and without the minimum image of the repulsive pairs (the same
 // for a whole molecule).
 template <int G, bool UNI, class XS>
-__device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, int lane,
-                                           int2 br, int2 ar, int abase, int acnt, int rcnt,
+__device__ __forceinline__ void bead_force(const DevSys& s, const XS& X, int i, int m1, long long n,
+                                           int lane, int2 br, int2 ar, int abase, int acnt, int rcnt,
                                            float& fx, float& fy, float& fz, bool& fene_bad) {
-  if (s.grid[m1].wrap_list)
-    bead_force_w<G, UNI, true>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
+  if (list_image_taken(s, m1, n))
+    bead_force_w<G, UNI, true>(s, X, i, m1, n, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
   else
-    bead_force_w<G, UNI, false>(s, X, i, m1, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
+    bead_force_w<G, UNI, false>(s, X, i, m1, n, lane, br, ar, abase, acnt, rcnt, fx, fy, fz, fene_bad);
 }
 
 }  // namespace sop
