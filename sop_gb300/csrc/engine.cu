@@ -318,6 +318,23 @@ struct SopCtx {
 
 static SopCtx* C(void* p) { return static_cast<SopCtx*>(p); }
 
+// Makes the context's device current for a call and gives the caller's back: a
+// kernel launched into a stream of another device than the current one fails.
+class OnDevice {
+ public:
+  explicit OnDevice(const SopCtx* ctx) {
+    if (cudaGetDevice(&was_) != cudaSuccess || was_ == ctx->P.device) was_ = -1;
+    else cudaSetDevice(ctx->P.device);
+  }
+  ~OnDevice() {
+    if (was_ >= 0) cudaSetDevice(was_);
+  }
+  OnDevice(const OnDevice&) = delete;
+
+ private:
+  int was_ = -1;
+};
+
 int grow_nl_keep(SopCtx* ctx, long long stride);
 
 #define CK(call)                                         \
@@ -2099,6 +2116,7 @@ int sop_serve_submit(void* p, const sop_molecule* m, int* job) {
 int sop_serve_advance(void* p, int rounds) {
   if (!p || rounds < 0) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->served) return ctx->fail(SOP_ERR_ARG, "not a served context");
   for (int r = 0; r < rounds; ++r) {
     int rc = serve_round(ctx);
@@ -2172,6 +2190,7 @@ int sop_upload_topology(void* p, const sop_molecule* m) {
 int sop_upload_state(void* p, int mol, const float* pos, const float* unc_pos, const float* vel) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2208,6 +2227,7 @@ int sop_upload_state(void* p, int mol, const float* pos, const float* unc_pos, c
 int sop_step(void* p, long long nsteps) {
   if (!p || nsteps < 0) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = step_async(ctx, nsteps);
   if (rc) return rc;
@@ -2217,6 +2237,7 @@ int sop_step(void* p, long long nsteps) {
 int sop_step_async(void* p, long long nsteps) {
   if (!p || nsteps < 0) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   return step_async(ctx, nsteps);
 }
@@ -2224,6 +2245,7 @@ int sop_step_async(void* p, long long nsteps) {
 int sop_sync(void* p) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   ctx->queued = true;
   int rc = sync_checked(ctx);
@@ -2235,6 +2257,7 @@ int sop_sync(void* p) {
 int sop_launch_stage(void* p, int stage, int koff) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   ctx->queued = true;
   switch (stage) {
@@ -2259,6 +2282,7 @@ int sop_launch_stage(void* p, int stage, int koff) {
 int sop_update_neighbor_list(void* p, long long* nnl_att, long long* nnl_rep) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2280,6 +2304,7 @@ int sop_update_neighbor_list(void* p, long long* nnl_att, long long* nnl_rep) {
 int sop_update_pair_list(void* p, long long* nil_att, long long* nil_rep) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2302,6 +2327,7 @@ int sop_update_pair_list(void* p, long long* nil_att, long long* nil_rep) {
 int sop_force_eval(void* p) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2314,6 +2340,7 @@ int sop_force_eval(void* p) {
 int sop_set_noise(void* p, const float* normals) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2337,6 +2364,7 @@ int sop_set_noise(void* p, const float* normals) {
 int sop_download(void* p, int mol, float* pos, float* unc_pos, float* vel, float* force) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2368,6 +2396,7 @@ int sop_download_list(void* p, int mol, int which, long long cap, int* i_out, in
                       float* r0_out, long long* count) {
   if (!p || which < 0 || which > 3) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2434,6 +2463,7 @@ int sop_download_list(void* p, int mol, int which, long long cap, int* i_out, in
 int sop_list_sizes(void* p, long long* out) {
   if (!p || !out) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2451,6 +2481,7 @@ int sop_list_sizes(void* p, long long* out) {
 int sop_download_all(void* p, float* unc_pos) {
   if (!p || !unc_pos) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
@@ -2471,6 +2502,7 @@ int sop_download_all(void* p, float* unc_pos) {
 int sop_download_all_async(void* p, float* unc_pos, long long* ticket) {
   if (!p || !unc_pos || !ticket) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   ctx->queued = true;
   if (!ctx->copy_stream) {
@@ -2507,6 +2539,7 @@ int sop_download_all_async(void* p, float* unc_pos, long long* ticket) {
 int sop_download_wait(void* p, long long ticket) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (ticket < 0 || ticket >= ctx->next_ticket || !ctx->copy_stream)
     return ctx->fail(SOP_ERR_ARG, "no such download");
   // a buffer's event is re-recorded by the download two tickets later, whose
@@ -2523,6 +2556,7 @@ int sop_download_wait(void* p, long long ticket) {
 int sop_energy(void* p, int mol, double* terms) {
   if (!p || !terms) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2538,6 +2572,7 @@ int sop_energy(void* p, int mol, double* terms) {
 int sop_observables(void* p, int mol, double* out) {
   if (!p || !out) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2554,6 +2589,7 @@ int sop_observables(void* p, int mol, double* out) {
 int sop_molecule_status(void* p, int mol, int* status, long long* step) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
   rc = sync_checked(ctx);
@@ -2586,6 +2622,7 @@ static int copy_out_ckpt(SopCtx* ctx, const std::vector<char>& blob, void* buf, 
 int sop_checkpoint(void* p, int mol, void* buf, long long cap, long long* size) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (ctx->served) return ctx->fail(SOP_ERR_ARG, "served contexts use sop_serve_checkpoint");
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
@@ -2600,6 +2637,7 @@ int sop_checkpoint(void* p, int mol, void* buf, long long cap, long long* size) 
 int sop_restore(void* p, int mol, const void* buf, long long size) {
   if (!p || !buf) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (ctx->served) return ctx->fail(SOP_ERR_ARG, "served contexts use sop_serve_resume");
   int rc = check_mol(ctx, mol);
   if (rc) return rc;
@@ -2630,6 +2668,7 @@ int sop_restore(void* p, int mol, const void* buf, long long size) {
 int sop_serve_checkpoint(void* p, int job, void* buf, long long cap, long long* size) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->served) return ctx->fail(SOP_ERR_ARG, "not a served context");
   if (job < 0 || job >= (int)ctx->jobs.size()) return ctx->fail(SOP_ERR_NOT_FOUND, "unknown job");
   if (ctx->jobs[job].state != Job::ACTIVE) return ctx->fail(SOP_ERR_ARG, "job is not running");
@@ -2707,6 +2746,7 @@ int sop_check_step_barrier(void* p, int missing, double timeout_s, int* timed_ou
   if (!p || !timed_out || missing < 0 || !(timeout_s > 0.0) || timeout_s > 10.0)
     return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
+  OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   int rc = sync_checked(ctx);
   if (rc) return rc;
