@@ -1218,17 +1218,37 @@ int install(SopCtx* ctx, int slot, HostMol& hm, long long step0) {
   return upload_staged(ctx, S);
 }
 
-// Returns the pool ranges of molecule slot `slot`, which the device no longer
-// uses (k_retire).
-void release_slot(SopCtx* ctx, int slot) {
-  HostMol& hm = ctx->mols[slot];
+void release_ranges(SopCtx* ctx, HostMol& hm) {
   ctx->bead_alloc.release(hm.start, hm.n);
   ctx->bond_alloc.release(hm.off_b, 2LL * (long long)hm.bi.size());
   ctx->ang_alloc.release(hm.off_a, 2LL * (long long)hm.ai.size());
   ctx->nat_alloc.release(hm.off_n, 2LL * (long long)hm.ni.size());
+  hm.start = -1;
+}
+
+// Returns the pool ranges of molecule slot `slot`, which the device no longer
+// uses (k_retire).
+void release_slot(SopCtx* ctx, int slot) {
+  release_ranges(ctx, ctx->mols[slot]);
   ctx->mc[slot] = MolConst{};
-  hm = HostMol();
+  ctx->mols[slot] = HostMol();
   ctx->free_slots.push_back(slot);
+}
+
+// Frees slot `slot` of a molecule that could not be admitted, which goes back to
+// `mol` (the stream idle).
+int vacate(SopCtx* ctx, int slot, HostMol& mol) {
+  mol = std::move(ctx->mols[slot]);
+  ctx->mols[slot] = HostMol();
+  ctx->free_slots.push_back(slot);
+  if (mol.start < 0) return SOP_OK;  // it took no ranges
+  const int start = mol.start;
+  release_ranges(ctx, mol);
+  const MolConst off{};
+  ctx->mc[slot] = off;
+  CK(cudaMemcpy(ctx->dmol + slot, &off, sizeof off, cudaMemcpyHostToDevice));
+  CK(cudaMemset(ctx->s.mol_of + start, 0xff, sizeof(int) * (size_t)mol.n));
+  return SOP_OK;
 }
 
 // Molecules on their way into their slots, their rows in the pinned buffer.
@@ -1985,6 +2005,7 @@ static int serve_round(SopCtx* ctx) {
   for (auto it = ctx->queue.begin(); it != ctx->queue.end() && looked < 64 && !ctx->free_slots.empty();) {
     Job& jb = ctx->jobs[*it];
     const int slot = ctx->free_slots.back();
+    ctx->free_slots.pop_back();
     ctx->mols[slot] = std::move(jb.mol);
     for (int t : ctx->mols[slot].types)
       if (t != 1 && ctx->s.uniform_type) {
@@ -1994,22 +2015,26 @@ static int serve_round(SopCtx* ctx) {
     const bool resumed = !jb.resume.empty();
     rc = resumed ? install(ctx, slot, ctx->mols[slot], jb.resume_step)
                  : collect_arrival(ctx, slot, ctx->mols[slot], -(long long)ctx->P.nnlup, arrivals);
-    if (rc == SOP_ERR_CAPACITY) {
-      jb.mol = std::move(ctx->mols[slot]);
-      ctx->mols[slot] = HostMol();
-      ++it;
-      ++looked;
-      continue;
-    }
-    if (rc) return rc;
-    if (resumed) {
-      // the job continues at its checkpoint's step, with its state and lists
+    const bool no_room = rc == SOP_ERR_CAPACITY;
+    // the job continues at its checkpoint's step, with its state and lists
+    if (!rc && resumed)
       rc = restore_into(ctx, slot, jb.resume.data(), (long long)jb.resume.size());
-      if (rc) return rc;
+    if (rc) {  // the job stays queued as it was
+      const std::string why = ctx->err;
+      vacate(ctx, slot, jb.mol);
+      if (no_room) {
+        ++it;
+        ++looked;
+        continue;
+      }
+      flush_arrivals(ctx, arrivals);  // those admitted before it are in their slots
+      ctx->err = why;
+      return rc;
+    }
+    if (resumed) {
       jb.resume.clear();
       jb.resume.shrink_to_fit();
     }
-    ctx->free_slots.pop_back();
     ctx->slot_job[slot] = *it;
     jb.slot = slot;
     jb.state = Job::ACTIVE;
