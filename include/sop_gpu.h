@@ -281,6 +281,14 @@ int sop_tuning(void* ctx, int* lanes, float* ms);
  * rebuilds in one cooperative launch, 4 the same in one block). */
 int sop_step_form(void* ctx, int* lanes, int* form);
 
+/* Which kernel takes the steps of a context whose reads are staged in shared
+ * memory: kind 1 tiles of consecutive beads, 2 pair-list rebuild and step in
+ * one launch, 0 the steps are not staged; its lanes per bead; for kind 1 the
+ * tiles and how many of them gather from global memory because their lists do
+ * not fit (those of the last pair-list rebuild), else 0.  Out pointers may be
+ * NULL. */
+int sop_staged(void* ctx, int* kind, int* lanes, int* tiles, int* gathered);
+
 /* The per-size-bucket tiling of the step (sop_params.step_buckets): *tiled
  * receives 1 when the tiled step is in use; per bucket (< 200, 200-599,
  * >= 600 beads) the lanes per bead and form chosen and the beads it holds

@@ -2767,6 +2767,27 @@ int sop_step_form(void* p, int* lanes, int* form) {
   return SOP_OK;
 }
 
+int sop_staged(void* p, int* kind, int* lanes, int* tiles, int* gathered) {
+  if (!p) return SOP_ERR_ARG;
+  SopCtx* ctx = C(p);
+  OnDevice on(ctx);
+  if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
+  const int n = ctx->tiles.beads ? ctx->tiles.ntile : 0;
+  if (kind) *kind = n ? 1 : ctx->pair_step ? 2 : 0;
+  if (lanes) *lanes = n ? 256 / ctx->tiles.beads : ctx->pair_step;
+  if (tiles) *tiles = n;
+  if (gathered) {
+    *gathered = 0;
+    if (!n) return SOP_OK;
+    int rc = sync_checked(ctx);
+    if (rc) return rc;
+    std::vector<int> cnt(n);
+    CK(cudaMemcpy(cnt.data(), ctx->tiles.cnt, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
+    for (int c : cnt) *gathered += c < 0;
+  }
+  return SOP_OK;
+}
+
 int sop_check_step_barrier(void* p, int missing, double timeout_s, int* timed_out) {
   if (!p || !timed_out || missing < 0 || !(timeout_s > 0.0) || timeout_s > 10.0)
     return SOP_ERR_ARG;

@@ -143,6 +143,7 @@ def lib() -> ctypes.CDLL:
                                      ctypes.POINTER(ctypes.c_double)]),
             "sop_serve_stats": (I, [V, V]),
             "sop_step_form": (I, [V, ctypes.POINTER(I), ctypes.POINTER(I)]),
+            "sop_staged": (I, [V] + [ctypes.POINTER(I)] * 4),
             "sop_step_window": (I, [V, ctypes.POINTER(I)]),
             "sop_step_buckets": (I, [V, ctypes.POINTER(I), V, V, V, V]),
             "sop_check_step_barrier": (I, [V, I, ctypes.c_double, ctypes.POINTER(I)]),
@@ -413,6 +414,16 @@ class Engine:
         return {"lanes_per_bead": g.value, "form": form.value, "window": win.value,
                 "buckets": buckets,
                 "ms": {str(k): float(v) for k, v in zip((2, 4, 8, 16), ms)}}
+
+    def staged(self) -> dict:
+        """Which kernel takes the steps of a staged context (sop_staged): kind
+        None, "tiles" or "pair list and step"; lanes per bead; tiles and how
+        many of them gather from global memory."""
+        v = [ctypes.c_int() for _ in range(4)]
+        self._check(lib().sop_staged(self.h, *map(ctypes.byref, v)), self.h)
+        kind, lanes, tiles, gathered = (x.value for x in v)
+        return {"kind": (None, "tiles", "pair list and step")[kind], "lanes": lanes, "tiles": tiles,
+                "gathered": gathered}
 
     def check_step_barrier(self, missing: int, timeout_s: float) -> bool:
         """Runs the persistent step's device-wide barrier with `missing`

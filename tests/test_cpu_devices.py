@@ -48,7 +48,7 @@ def serve():
     srv.advance(2)
 
 calls = dict(
-    restore=restore, download=lambda: [e.download(k) for k in (0, 1)], status=lambda: e.status(0),
+    staged=e.staged, restore=restore, download=lambda: [e.download(k) for k in (0, 1)], status=lambda: e.status(0),
     energy=lambda: e.energy(1), observables=lambda: e.observables(0),
     upload=lambda: [e.upload_state(k, q.xyz, vel=np.zeros_like(q.xyz)) for k, q in ((0, m), (1, big))],
     step=lambda: e.step(73), step_async=lambda: e.step_async(20), sync=e.sync,
