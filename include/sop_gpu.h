@@ -283,11 +283,11 @@ int sop_step_form(void* ctx, int* lanes, int* form);
 
 /* Which kernel takes the steps of a context whose reads are staged in shared
  * memory: kind 1 tiles of consecutive beads, 2 pair-list rebuild and step in
- * one launch, 0 the steps are not staged; its lanes per bead; for kind 1 the
- * tiles and how many of them gather from global memory because their lists do
- * not fit (those of the last pair-list rebuild), else 0.  Out pointers may be
- * NULL. */
-int sop_staged(void* ctx, int* kind, int* lanes, int* tiles, int* gathered);
+ * one launch, 0 the steps are not staged; its lanes per bead; for kind 2 the
+ * beads a block stages its molecules in (0: it gathers from global memory); for
+ * kind 1 the tiles and how many of them gather because their lists do not fit
+ * (those of the last pair-list rebuild).  Out pointers may be NULL. */
+int sop_staged(void* ctx, int* kind, int* lanes, int* window, int* tiles, int* gathered);
 
 /* The per-size-bucket tiling of the step (sop_params.step_buckets): *tiled
  * receives 1 when the tiled step is in use; per bucket (< 200, 200-599,

@@ -54,8 +54,8 @@ cudaError_t launch_step_tile(const DevSys& s, const TileSet& ts, int koff, bool 
                              cudaStream_t st);
 cudaError_t launch_pl_tile(const DevSys& s, const TileSet& ts, int koff, bool only_tables,
                            cudaStream_t st);
-cudaError_t launch_pair_step(const DevSys& s, int lanes, int koff, bool early, int max_mol,
-                             cudaStream_t st);
+cudaError_t plan_pair_step(const DevSys& s, int lanes, int max_mol, PairPlan* p);
+cudaError_t launch_pair_step(const DevSys& s, const PairPlan& p, int koff, bool early, cudaStream_t st);
 void launch_gather_current(const DevSys& s, float* out, int* flag_out, cudaStream_t st);
 int energy_blocks(int mol_n);
 void launch_observables(const DevSys& s, int mol_start, int mol_n, int m, int nnat,
@@ -206,7 +206,7 @@ struct SopCtx {
   bool persist = false;       // steps between list rebuilds in one cooperative launch
   bool one_block = false;     // steps between list rebuilds in one block
   TileSet tiles{};            // tables of the tile step (tiles.beads 0: not used)
-  int pair_step = 0;          // lanes per bead of pair-list rebuild and step in one launch (0: apart)
+  PairPlan pair{};            // pair-list rebuild and step in one launch (pair.lanes 0: apart)
   // tiled form: per-molecule tiles, lanes and form chosen per size bucket
   bool tiled = false;
   int4* d_tiles = nullptr;    // {first bead, end bead, lanes, two-kernel form}
@@ -348,7 +348,7 @@ namespace {
 int graph_steps(const SopCtx* ctx);
 
 // The steps run staged (kernels_tile.cu).
-bool staged(const SopCtx* ctx) { return ctx->tiles.beads || ctx->pair_step; }
+bool staged(const SopCtx* ctx) { return ctx->tiles.beads || ctx->pair.lanes; }
 
 // The rows of the molecule whose beads are o .. o + n - 1 in the repulsive
 // neighbour list (r = 0) or pair list (r = 1), in row order, every entry as an
@@ -559,7 +559,7 @@ void rebuild_pairs(SopCtx* ctx, const DevSys& s, int koff) {
 // Copies the coordinates to where k_pair_step reads the last step's: after
 // every change of them other than by its own steps.
 int keep_last(SopCtx* ctx) {
-  if (!ctx->pair_step) return SOP_OK;
+  if (!ctx->pair.lanes) return SOP_OK;
   for (int b = 0; b < 2; ++b)
     CK(cudaMemcpyAsync(ctx->s.xl[b], ctx->s.x[b], sizeof(float4) * (size_t)ctx->s.nbead,
                        cudaMemcpyDeviceToDevice, ctx->stream));
@@ -578,36 +578,40 @@ int keep_last(SopCtx* ctx) {
 // step (factor cut-offs): 128 beads 389 / 570, 2,000 529 / 686, 8,000 682 / 980,
 // 16,000 833 / 1,188.
 constexpr long long kStagedBeads = 16384, kStagedSmall = 8192;
-// With short rows the second lasts as long as its blocks (8 lanes a bead, four
-// blocks an SM) run as one wave: 18,000 beads 977 -> 715 us, 20,000 extended 502
-// / 493, 24,000 1,108 / 1,097, 120 molecules of 200-450 beads 1,977 / 2,150.
-// With long ones it loses past kStagedBeads: 80 molecules of 100-1,500 beads at
-// 32 A 2,384 / 2,926.
-constexpr long long kPairBeads = 152 * 4 * 32, kPairShortRow = 512;
+// With short rows the second lasts as long as its blocks at 8 lanes a bead run as
+// one wave (PairPlan::wave; four on each of 152 SMs: 19,456 beads): not staged /
+// staged 17,000 beads 859 / 628 us, 19,456 beads 881 / 641 (at 16 lanes 983 / 886),
+// 13 molecules of 1,495 864 / 672, 41 of 450 804 / 610, 90 of 200 766 / 566, but 24,000
+// beads 1,097 / 1,108, 120 molecules of 200-450 beads 1,977 / 2,150.  With long ones it loses
+// past kStagedBeads: 80 molecules of 100-1,500 beads at 32 A 2,384 / 2,926.
+constexpr long long kPairShortRow = 512;
 int alloc_staged(SopCtx* ctx) {
   const sop_params& P = ctx->P;
   TileSet& ts = ctx->tiles;
   ts = TileSet{};
-  ctx->pair_step = 0;
+  ctx->pair = PairPlan{};
   const int lanes = lanes_for(ctx);
   const bool pair = P.nplup <= 1, short_rows = ctx->s.nl_stride <= kPairShortRow;
   if (ctx->served || P.step_split > 1 || P.step_window > 0 || P.step_buckets > 0 ||
-      ctx->s.nbead > (pair && short_rows ? kPairBeads : kStagedBeads))
+      (lanes && lanes != 8 && lanes != 16))
     return SOP_OK;
   if (pair) {
-    if (lanes && lanes != 8 && lanes != 16) return SOP_OK;
-    for (int b = 0; b < 2; ++b) {
-      ctx->s.xl[b] = ctx->dalloc<float4>(ctx->s.nbead);
-      if (!ctx->s.xl[b]) return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
-    }
     // 8 lanes for larger contexts, but not for long rows (up to 512 entries at
     // the factor cut-offs, 1,088 at 32 A): us per 50 steps with 8 / 16 lanes,
     // 8,000 beads 708 / 682, 12,000 758 / 901; 10,900 beads at 32 A 1,354 / 1,096
     const bool eight = ctx->s.nbead > kStagedSmall && short_rows;
-    ctx->pair_step = lanes ? lanes : eight ? 8 : 16;
+    PairPlan plan{}, widest{};
+    CK(plan_pair_step(ctx->s, lanes ? lanes : eight ? 8 : 16, ctx->w.max_mol, &plan));
+    CK(plan_pair_step(ctx->s, 8, ctx->w.max_mol, &widest));
+    if (ctx->s.nbead > std::max(kStagedBeads, short_rows ? widest.wave : 0)) return SOP_OK;
+    for (int b = 0; b < 2; ++b) {
+      ctx->s.xl[b] = ctx->dalloc<float4>(ctx->s.nbead);
+      if (!ctx->s.xl[b]) return ctx->fail(SOP_ERR_ALLOC, "device allocation failed");
+    }
+    ctx->pair = plan;
     return keep_last(ctx);
   }
-  if (lanes && lanes != 8 && lanes != 16) return SOP_OK;
+  if (ctx->s.nbead > kStagedBeads) return SOP_OK;
   const int tb = lanes ? 256 / lanes : ctx->s.nbead <= kStagedSmall ? 16 : 32;
   const size_t n = ((size_t)ctx->s.nbead + tb - 1) / tb;
   ts.ntile = (int)n;
@@ -680,7 +684,7 @@ int rebuilds_before(const sop_params& P, long long n) {
 void enqueue_block(SopCtx* ctx, long long s0, int count) {
   int run0 = 0;  // first step of the current run without rebuilds
   int base = 0;  // steps of the block the clocks already count
-  if (ctx->pair_step) {  // the pair-list rebuild precedes every step, in its launch
+  if (ctx->pair.lanes) {  // the pair-list rebuild precedes every step, in its launch
     bool early = false;  // a step is the launch before
     for (int k = 0; k < count; ++k) {
       if (rebuilds_before(ctx->P, s0 + 1 + k) & 1) {
@@ -689,7 +693,7 @@ void enqueue_block(SopCtx* ctx, long long s0, int count) {
         launch_nl_rebuild(ctx->s, ctx->w, 0, ctx->stream);
         early = false;
       }
-      launch_pair_step(ctx->s, ctx->pair_step, k - base, early, ctx->w.max_mol, ctx->stream);
+      launch_pair_step(ctx->s, ctx->pair, k - base, early, ctx->stream);
       early = true;
     }
     launch_advance(ctx->s, count - base, ctx->stream);
@@ -2287,7 +2291,7 @@ int sop_launch_stage(void* p, int stage, int koff) {
   ctx->queued = true;
   switch (stage) {
     case 0:
-      if (ctx->pair_step) CK(launch_pair_step(ctx->s, ctx->pair_step, koff, false, ctx->w.max_mol, ctx->stream));
+      if (ctx->pair.lanes) CK(launch_pair_step(ctx->s, ctx->pair, koff, false, ctx->stream));
       else launch_steps(ctx, koff, 1);
       break;
     case 1: rebuild_pairs(ctx, ctx->s, koff); break;
@@ -2762,19 +2766,20 @@ int sop_tuning(void* p, int* lanes, float* ms) {
 int sop_step_form(void* p, int* lanes, int* form) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
-  if (lanes) *lanes = ctx->tiles.beads ? 256 / ctx->tiles.beads : ctx->pair_step ? ctx->pair_step : ctx->G;
+  if (lanes) *lanes = ctx->tiles.beads ? 256 / ctx->tiles.beads : ctx->pair.lanes ? ctx->pair.lanes : ctx->G;
   if (form) *form = staged(ctx) ? 1 : ctx->one_block ? 4 : ctx->persist ? 3 : ctx->split ? 2 : 1;
   return SOP_OK;
 }
 
-int sop_staged(void* p, int* kind, int* lanes, int* tiles, int* gathered) {
+int sop_staged(void* p, int* kind, int* lanes, int* window, int* tiles, int* gathered) {
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
   OnDevice on(ctx);
   if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   const int n = ctx->tiles.beads ? ctx->tiles.ntile : 0;
-  if (kind) *kind = n ? 1 : ctx->pair_step ? 2 : 0;
-  if (lanes) *lanes = n ? 256 / ctx->tiles.beads : ctx->pair_step;
+  if (kind) *kind = n ? 1 : ctx->pair.lanes ? 2 : 0;
+  if (lanes) *lanes = n ? 256 / ctx->tiles.beads : ctx->pair.lanes;
+  if (window) *window = ctx->pair.win;
   if (tiles) *tiles = n;
   if (gathered) {
     *gathered = 0;

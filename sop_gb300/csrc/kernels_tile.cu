@@ -23,6 +23,7 @@
 // The per-entry and per-bead arithmetic is k_step's (step_dev.cuh) in the same
 // order, so every bit is the same.  A tile whose lists do not fit (long rows, a
 // dense structure) gathers as k_step does.
+#include <algorithm>
 #include <type_traits>
 
 #include "lists_dev.cuh"
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_step_tile(DevSys s, TileSet
 // way through L2 took 16 us a step at 1,531 beads.
 // A block's molecules (from its first bead's to its last bead's) are staged in
 // shared memory where they fit in `win` beads, else gathered from L2.
-constexpr int kPairWindow = 1600; // most staged beads
+constexpr int kPairWindow = 1600; // most staged beads (two sets: 51 KB, three blocks of 16 lanes an SM)
 constexpr int kPairRep = 256;     // entries of a repulsive row kept in shared memory
 constexpr int kPairAtt = 32;      // and of an attractive one (past them: read from L2)
 template <int G, bool UNI>
@@ -530,24 +531,57 @@ cudaError_t launch_pl_tile(const DevSys& s, const TileSet& ts, int koff, bool on
                         : pl_tb<32>(s, ts, koff, only_tables, st);
 }
 
-// The pair-list rebuild and the step after it, 8 or 16 lanes a bead; max_mol:
-// beads of the context's largest molecule.
+// The pair-list rebuild and the step after it, 8 or 16 lanes a bead.
+template <int G>
+static auto pair_kernel(const DevSys& s) { return s.uniform_type ? k_pair_step<G, true> : k_pair_step<G, false>; }
+
+static size_t pair_smem(int win) { return 2 * (size_t)win * sizeof(float4); }
+
 template <int G>
 static cudaError_t pair_g(const DevSys& s, int koff, bool early, int win, cudaStream_t st) {
-  auto kernel = s.uniform_type ? k_pair_step<G, true> : k_pair_step<G, false>;
+  auto kernel = pair_kernel<G>(s);
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             2 * kPairWindow * (int)sizeof(float4));
+                                             (int)pair_smem(kPairWindow));
   if (e != cudaSuccess) return e;
   constexpr int beads = kTileThreads / G;
-  return launch_pdl_smem(kernel, (unsigned)((s.nlive + beads - 1) / beads), kTileThreads,
-                         2 * (size_t)win * sizeof(float4), st, s, koff, early ? 1 : 0, win);
+  return launch_pdl_smem(kernel, (unsigned)((s.nlive + beads - 1) / beads), kTileThreads, pair_smem(win), st,
+                         s, koff, early ? 1 : 0, win);
 }
 
-cudaError_t launch_pair_step(const DevSys& s, int lanes, int koff, bool early, int max_mol,
-                             cudaStream_t st) {
-  // two coordinate sets of up to 1,600 beads: two blocks per SM
+cudaError_t launch_pair_step(const DevSys& s, const PairPlan& p, int koff, bool early, cudaStream_t st) {
+  return p.lanes == 16 ? pair_g<16>(s, koff, early, p.win, st) : pair_g<8>(s, koff, early, p.win, st);
+}
+
+// The window takes shared memory, so fewer blocks are resident: it is used
+// where the context's blocks run in as many waves with it as without.  us per 50
+// steps with the window / without, factor cut-offs: one molecule of 800 beads 313 /
+// 344, 1,531 350 / 359, 10 of 400 343 / 352, at 32 A 6 of 1,200 655 / 782 and (two
+// waves both) 8 of 1,500 1,137 / 1,167; where it takes a wave more 5 of 1,600 729 /
+// 480, 20 of 800 797 / 605, 13 of 1,495 956 / 672, at 32 A 5 of 1,500 874 / 820.
+template <int G>
+static cudaError_t plan_g(const DevSys& s, int max_mol, PairPlan* p) {
+  auto kernel = pair_kernel<G>(s);
+  int dev = 0, sms = 0, with = 0, without = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(kPairWindow));
   const int win = max_mol > kPairWindow ? 0 : (max_mol + 256 < kPairWindow ? max_mol + 256 : kPairWindow);
-  return lanes == 16 ? pair_g<16>(s, koff, early, win, st) : pair_g<8>(s, koff, early, win, st);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with, kernel, kTileThreads, pair_smem(win));
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&without, kernel, kTileThreads, 0);
+  if (e != cudaSuccess) return e;
+  constexpr int beads = kTileThreads / G;
+  const long long blocks = (s.nlive + beads - 1) / beads;
+  auto waves = [&](int resident) { return (blocks - 1) / std::max(1LL, (long long)resident * sms); };
+  p->lanes = G;
+  p->win = waves(with) <= waves(without) ? win : 0;
+  p->wave = (long long)without * sms * beads;
+  return cudaSuccess;
+}
+
+cudaError_t plan_pair_step(const DevSys& s, int lanes, int max_mol, PairPlan* p) {
+  return lanes == 16 ? plan_g<16>(s, max_mol, p) : plan_g<8>(s, max_mol, p);
 }
 
 }  // namespace sop

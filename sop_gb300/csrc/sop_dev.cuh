@@ -154,6 +154,13 @@ __device__ __forceinline__ bool list_image_taken(const DevSys& s, int m, long lo
   return flag != 0 && flag != image_mark(n);
 }
 
+// How k_pair_step (kernels_tile.cu) is launched: lanes per bead (0: not used),
+// the window in beads, and the beads that run as one wave without a window.
+struct PairPlan {
+  int lanes, win;
+  long long wave;
+};
+
 // Tables of the tile step (kernels_tile.cu), rebuilt after every pair-list
 // rebuild; a tile is `beads` consecutive bead slots.
 constexpr int kTileCap = 2048;     // distinct beads a tile may touch

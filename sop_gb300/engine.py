@@ -143,7 +143,7 @@ def lib() -> ctypes.CDLL:
                                      ctypes.POINTER(ctypes.c_double)]),
             "sop_serve_stats": (I, [V, V]),
             "sop_step_form": (I, [V, ctypes.POINTER(I), ctypes.POINTER(I)]),
-            "sop_staged": (I, [V] + [ctypes.POINTER(I)] * 4),
+            "sop_staged": (I, [V] + [ctypes.POINTER(I)] * 5),
             "sop_step_window": (I, [V, ctypes.POINTER(I)]),
             "sop_step_buckets": (I, [V, ctypes.POINTER(I), V, V, V, V]),
             "sop_check_step_barrier": (I, [V, I, ctypes.c_double, ctypes.POINTER(I)]),
@@ -417,13 +417,13 @@ class Engine:
 
     def staged(self) -> dict:
         """Which kernel takes the steps of a staged context (sop_staged): kind
-        None, "tiles" or "pair list and step"; lanes per bead; tiles and how
-        many of them gather from global memory."""
-        v = [ctypes.c_int() for _ in range(4)]
+        None, "tiles" or "pair list and step"; lanes per bead; the window of
+        a block in beads; tiles and how many of them gather."""
+        v = [ctypes.c_int() for _ in range(5)]
         self._check(lib().sop_staged(self.h, *map(ctypes.byref, v)), self.h)
-        kind, lanes, tiles, gathered = (x.value for x in v)
-        return {"kind": (None, "tiles", "pair list and step")[kind], "lanes": lanes, "tiles": tiles,
-                "gathered": gathered}
+        kind, lanes, window, tiles, gathered = (x.value for x in v)
+        return {"kind": (None, "tiles", "pair list and step")[kind], "lanes": lanes, "window": window,
+                "tiles": tiles, "gathered": gathered}
 
     def check_step_barrier(self, missing: int, timeout_s: float) -> bool:
         """Runs the persistent step's device-wide barrier with `missing`

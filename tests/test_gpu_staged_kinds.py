@@ -1,6 +1,7 @@
 """Which contexts the staged steps take (Engine.staged): the comparisons of
 test_gpu_staged.py and test_gpu_pair_rows.py are of the kernels they name, both
 kinds of tile among them, and the edges of the ranges lie where they are said to."""
+import numpy as np
 import pytest
 
 from sop_gb300 import engine, system
@@ -56,3 +57,29 @@ def test_edges_of_the_ranges(n, nplup, kind, lanes):
 def test_what_the_parameters_ask_for_instead(kw, nplup):
     with one(500, nplup=nplup, **kw) as e:
         assert e.staged()["kind"] is None
+
+
+@pytest.mark.parametrize("count,n,lanes,window", [
+    (1, 1344, 16, 1600), (1, 1600, 16, 1600), (1, 1601, 16, 0), (10, 400, 16, 656),
+    # 304 blocks at three an SM, then more blocks than are resident with a window
+    (6, 800, 16, 1056), (5, 1600, 16, 0), (20, 800, 8, 0), (13, 1495, 8, 0), (41, 450, 8, 0)])
+def test_window_while_the_blocks_are_resident(count, n, lanes, window):
+    """Launches of one wave with their window (152 SMs) take it; where it keeps
+    blocks from being resident they gather.  The steps are the same bits."""
+    states = []
+    for kw in ({}, dict(step_split=2, lanes_per_bead=4)):
+        if (n, 0) not in _MOLS:
+            _MOLS[n, 0] = system.generate(n, 3)
+        m = _MOLS[n, 0]
+        e = engine.Engine(engine.default_params(h=0.02, zeta=0.05, **kw))
+        for k in range(count):
+            e.add(m, m.xyz, T=0.6, traj=k)
+        e.commit()
+        if not kw:
+            s = e.staged()
+            assert (s["kind"], s["lanes"], s["window"]) == ("pair list and step", lanes, window)
+        e.step(53)
+        states.append([e.download_all()] + [e.download(count - 1)[k] for k in ("vel", "force")])
+        e.close()
+    for a, b in zip(*states):
+        assert np.array_equal(a, b)
