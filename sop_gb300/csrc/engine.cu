@@ -2775,7 +2775,6 @@ int sop_staged(void* p, int* kind, int* lanes, int* window, int* tiles, int* gat
   if (!p) return SOP_ERR_ARG;
   SopCtx* ctx = C(p);
   OnDevice on(ctx);
-  if (!ctx->committed) return ctx->fail(SOP_ERR_ARG, "context not committed");
   const int n = ctx->tiles.beads ? ctx->tiles.ntile : 0;
   if (kind) *kind = n ? 1 : ctx->pair.lanes ? 2 : 0;
   if (lanes) *lanes = n ? 256 / ctx->tiles.beads : ctx->pair.lanes;

@@ -412,7 +412,7 @@ class Engine:
                                         "form": int(bf[k])}
                                  for k, name in enumerate(("<200", "200-599", ">=600"))}}
         return {"lanes_per_bead": g.value, "form": form.value, "window": win.value,
-                "buckets": buckets,
+                "buckets": buckets, "staged": self.staged()["kind"],
                 "ms": {str(k): float(v) for k, v in zip((2, 4, 8, 16), ms)}}
 
     def staged(self) -> dict:
@@ -460,12 +460,16 @@ def matched_params(params: Params, tuned: dict) -> Params:
     """A copy of `params` fixed to the lanes per bead and the step form the
     tuner chose for a context (Engine.tuning()), without the size-bucket
     tiles.  Unchanged when it chose the tiles, which the parameters cannot
-    fix, or the one-block form, which the tuner tries only for contexts of up
-    to 2,048 beads.  The window stays as the parameters give it: the tuner uses
-    one only where they fix it."""
+    fix, or the one-block form, which is for contexts of up to 2,048 beads.  A
+    context whose steps are staged passes its form on but not its lanes, which go
+    by its own size: us per 50 steps with / without them, two contexts of 8,000 and
+    8,400 beads 693 / 637; 16,000 and 17,600 937 (form and tuned lanes; with neither
+    1,048, the second one in two kernels).  The window stays as the parameters
+    give it: the tuner uses one only where they fix it."""
     q = Params.from_buffer_copy(params)
     if not tuned["buckets"]["tiled"] and tuned["form"] in (1, 2):
-        q.lanes_per_bead = tuned["lanes_per_bead"]
+        if not tuned.get("staged"):
+            q.lanes_per_bead = tuned["lanes_per_bead"]
         q.step_split = tuned["form"]
         q.step_buckets = -1
     return q
