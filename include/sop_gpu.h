@@ -86,12 +86,15 @@ typedef struct sop_params {
                          in one cooperative launch (a device-wide barrier
                          between steps), 4 the same in one block of 1,024
                          threads (block barriers), 0 chosen at commit: form 1
-                         for plain and batched contexts of up to 16,384 bead
-                         slots (with 0 or 1, and 0, 8 or 16 lanes per bead, its
-                         reads are then staged in shared memory), by timing
-                         for larger ones (served contexts: 2 above 65,536 bead
-                         slots in use, else 1).  Every form gives the same
-                         bits. */
+                         where the steps are staged (sop_staged), by timing
+                         elsewhere (served contexts: 2 above 65,536 bead slots
+                         in use, else 1).  With 0 or 1, 0, 8 or 16 lanes per
+                         bead, no window and no size buckets asked for, plain
+                         and batched contexts stage their steps up to 16,384
+                         bead slots, and where a pair list precedes every step
+                         and rows are short (up to 512 entries) as far as their
+                         blocks run as one wave (19,456 on a GB300).  Every
+                         form gives the same bits. */
   int step_window;    /* shared-memory window of the step, in beads: each step
                          block stages the coordinates of its beads' molecules
                          (up to this many beads) and gathers partners from
@@ -272,9 +275,11 @@ int sop_molecule_status(void* ctx, int mol, int* status, long long* step);
 int sop_memory(void* ctx, int mol, long long* ctx_bytes, long long* mol_bytes);
 
 /* Lanes per bead the step kernel uses (chosen at sop_commit by timing 2, 4, 8
- * and 16 unless sop_params.lanes_per_bead fixed it) and the measured kernel
- * times in ms for those four candidates (0 when not tuned).  Forces are
- * bit-identical for every choice. */
+ * and 16 unless sop_params.lanes_per_bead fixed it, or by the context's size
+ * where its steps are staged, sop_staged) and the measured kernel times in ms
+ * of the plain step kernel for those four candidates (0 when not tuned; a
+ * staged context evaluates forces outside its steps with the fastest).  Forces
+ * are bit-identical for every choice. */
 int sop_tuning(void* ctx, int* lanes, float* ms);
 /* The step's shape in use: lanes per bead, and its form (1 one kernel, 2 a
  * force kernel and a finish kernel, 3 persistent: the steps between two list

@@ -424,12 +424,12 @@ __global__ void k_advance(DevSys s, int steps) {
 // entries are independent and in flight together (one entry at a time, the
 // chain index -> coordinates -> divide took about 600 cycles an entry: 47 us
 // at 50,000 beads, 15 us at any small size).
-constexpr int kEnergyThreads = 128;
-constexpr int kTermBatch = 4;
-
 //
 // A molecule, or with a table one per blockIdx.y (the jobs that a served context
 // finishes together: a launch of 12 us for all of them instead of one each).
+constexpr int kEnergyThreads = 128;
+constexpr int kTermBatch = 4;
+
 __global__ void __launch_bounds__(kEnergyThreads) k_energy(DevSys s, EnergyJob job,
                                                             const RetireJob* __restrict__ jobs,
                                                             double* __restrict__ part) {

@@ -17,8 +17,10 @@
 //
 // What bounds k_step (kernels_step.cu) in a small context is latency: a chain
 // of about seven reads from L2 per bead and step, 8 us a step from 128 to 4,000
-// beads.  Here one round trip to L2 lies between the steps: 100 steps of 128
-// beads 725 -> 594 us, of 4,000 beads 1,057 -> 837 us, list rebuilds included.
+// beads.  Here one round trip to L2 lies between the steps.  us of a run and a
+// read of the state with k_step / staged, list rebuilds included: 100 steps of 128
+// beads 599 / 472, of 4,000 beads 884 / 788, extended 640 / 544; 50 steps of 1,531
+// beads with a list before every step 667 / 505.
 //
 // The per-entry and per-bead arithmetic is k_step's (step_dev.cuh) in the same
 // order, so every bit is the same.  A tile whose lists do not fit (long rows, a
