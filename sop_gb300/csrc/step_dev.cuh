@@ -191,13 +191,6 @@ __device__ __forceinline__ void complete_bead(const DevSys& s, int b, int m, flo
   inc = make_float4(__fmaf_rn(mc.a1, vi.x, __fmul_rn(mc.a2, fxx)),
                     __fmaf_rn(mc.a1, vi.y, __fmul_rn(mc.a2, fyy)),
                     __fmaf_rn(mc.a1, vi.z, __fmul_rn(mc.a2, fzz)), 0.f);
-  // moved too far for the minimum image to stay left out until the next look at
-  // the molecule's extent
-  const float far = fmaxf(fmaxf(fabsf(inc.x), fabsf(inc.y)), fabsf(inc.z));
-  if (!(far <= s.move_least) && !(far <= s.grid[m].move)) {
-    if (!s.grid[m].wrap) s.grid[m].wrap = image_mark(t.nb);
-    if (!s.grid[m].wrap_list) s.grid[m].wrap_list = image_mark(t.nb);
-  }
   s.incr[b] = inc;
   s.x[cur ^ 1][b] = make_float4(__fadd_rn(xo.x, inc.x), __fadd_rn(xo.y, inc.y),
                                 __fadd_rn(xo.z, inc.z), xo.w);
@@ -205,6 +198,13 @@ __device__ __forceinline__ void complete_bead(const DevSys& s, int b, int m, flo
   s.p[cur ^ 1][b] = make_float4(min_image(__fadd_rn(pi.x, inc.x), boxl),
                                 min_image(__fadd_rn(pi.y, inc.y), boxl),
                                 min_image(__fadd_rn(pi.z, inc.z), boxl), 0.f);
+  // moved too far for the minimum image to stay left out until the next look at
+  // the molecule's extent (after the stores: ahead of them 0.5% of the small steps)
+  const float far = fmaxf(fmaxf(fabsf(inc.x), fabsf(inc.y)), fabsf(inc.z));
+  if (!(far <= s.move_least) && !(far <= s.grid[m].move)) {
+    if (!s.grid[m].wrap) s.grid[m].wrap = image_mark(t.nb);
+    if (!s.grid[m].wrap_list) s.grid[m].wrap_list = image_mark(t.nb);
+  }
 }
 
 // Completes bead b (of molecule m) from its force sum fs; the step is the
