@@ -188,9 +188,10 @@ int sop_sync(void* ctx);
 
 /*
  * Queues one stage of the step loop at block offset koff, for timing and
- * profiling: 0 the fused force + Langevin step kernel, 1 the pair-list
- * rebuild, 2 the neighbour-list rebuild, 3 the end-of-block step advance
- * (count = koff).  Stages launched out of the loop's order leave the
+ * profiling: 0 the fused force + Langevin step kernel (with the pair-list
+ * rebuild that precedes it where both are one launch, sop_staged kind 2), 1
+ * the pair-list rebuild, 2 the neighbour-list rebuild, 3 the end-of-block step
+ * advance (count = koff).  Stages launched out of the loop's order leave the
  * trajectory undefined; the loop itself is sop_step.
  */
 int sop_launch_stage(void* ctx, int stage, int koff);

@@ -83,3 +83,13 @@ def test_window_while_the_blocks_are_resident(count, n, lanes, window):
         e.close()
     for a, b in zip(*states):
         assert np.array_equal(a, b)
+
+
+def test_form_that_is_reported():
+    """A default context of 128 beads, where the one-block form was once chosen:
+    staged, one kernel per step, 16 lanes; nothing is timed for its steps but the
+    plain kernel's force evaluations are."""
+    with engine.plain(system.generate(128, 0), params=engine.baseline_params()) as e:
+        t = e.tuning()
+        assert (t["staged"], t["form"], t["lanes_per_bead"]) == ("tiles", 1, 16)
+        assert all(v > 0 for v in t["ms"].values())
